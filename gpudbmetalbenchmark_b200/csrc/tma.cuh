@@ -68,6 +68,10 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       : "memory");
 }
 
+// Orders this thread's earlier shared-memory reads before bulk copies that overwrite the same
+// bytes (issued after a barrier, by any thread).
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 constexpr uint32_t kMbarPollLimit = 1u << 26;
 
 }  // namespace gpudb

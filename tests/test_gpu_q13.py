@@ -76,3 +76,24 @@ def test_q13_limits(engine, orc):
     with pytest.raises(capi.GpudbError) as e:
         run(engine, cu, od1, b"", b"requests")
     assert e.value.code == capi.E_INVALID
+
+
+@pytest.mark.parametrize("n_or", [1, 31, 32, 33, 257, 8 * 32 * 4 * 148 + 5])
+@pytest.mark.parametrize("w1,w2", [(b"special", b"requests"), (b"spe", b"requests"), (b"aaaaaaa", b"aaaaaaaaaaaaaaa")])
+def test_q13_tiles_and_candidates(engine, orc, n_or, w1, w2):
+    """Orders that fill no warp tile evenly, and comments whose candidates do not verify: word
+    prefixes before and after the words, at every alignment, and periodic words."""
+    rng = np.random.default_rng(n_or)
+    w1s, w2s = w1.decode(), w2.decode()
+    bits = [w1s, w2s, w1s[:-1], w1s[1:], w2s[:5], w2s[1:], "a", "aaaa", " ", "xy"]
+    pool = []
+    for _ in range(600):
+        s = "".join(bits[i] for i in rng.integers(0, len(bits), rng.integers(0, 12)))
+        pool.append(s[:79].encode())
+    for pad in range(80 - len(w1s + w2s)):
+        pool.append(b"q" * pad + w1 + w2)
+        pool.append(w1 + b"q" * pad + w2)
+    pool = np.array(pool, dtype="S80")
+    od = dict(cust_key=rng.integers(-1, 1001, n_or).astype(np.int32), comment=pool[rng.integers(0, len(pool), n_or)])
+    cu = dict(cust_key=np.arange(1000, dtype=np.int32))
+    assert run(engine, cu, od, w1, w2) == orc.q13(cu, od, w1, w2)
