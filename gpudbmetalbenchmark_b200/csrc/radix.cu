@@ -83,81 +83,137 @@ __global__ void __launch_bounds__(kPJThreads) partition_pairs_kernel(
   }
 }
 
-// Semi-join count: probe rows with at least one match. One 1024-thread block per partition
-// with a kPCCap-slot shared table (128 KB), so a partition of up to kPCChunk build keys is one
-// chunk and one 10-bit pass per side covers 15M build rows. Partitions whose build side needs
-// more than one chunk mark matches in `flags` (one byte per partitioned probe row) and count
-// them after the last chunk. Each thread keeps kPCRows build or probe keys in flight (the
-// kernel waits on those loads otherwise). A key's slot comes from the bits of its partition
-// hash above the `pbits` partition bits, so it is independent of the partition.
+// Semi-join count: probe rows with at least one match. One block per partition, a shared table
+// of the partition's build keys. key_hash32 is a bijection, so a key of the partition is named
+// by the hash bits above the `pbits` partition bits: kPCLog of them pick one of the
+// buckets and the rest (at most 15) are its tag, never 0 as stored. A bucket is four 16-bit
+// tags in one 64-bit word: a probe is one 8-byte shared load and a compare of four tags,
+// without a chain to walk (a linear-probing table of the keys ran a warp as long as the
+// longest chain of its 32 probes: 237 us for 7.5M build and 60M probe keys against 167 us; two
+// 512-thread blocks per SM with 2^13 buckets each need twice the partitions, which costs the
+// scatter 100 us more). A key whose bucket
+// is full (0.3% at one key a bucket) goes to the stash, a linear-probing set of full keys,
+// which only probes of full buckets look at.
+// A partition with more build rows than a chunk of kPCBuckets is joined chunk by chunk, its
+// matches marked in `flags` (one byte per partitioned probe row) and counted after the last
+// chunk; so is one whose keys overfill the stash (keys made to share buckets), in chunks that
+// the stash alone can hold.
 constexpr int kPCThreads = 1024;
-constexpr uint32_t kPCCap = 32768;
-constexpr uint32_t kPCChunk = kPCCap / 2;
-constexpr uint64_t kCountRowsPerPartition = 15360;   // average build keys per partition (<= kPCChunk with margin)
-constexpr int kPCRows = 16;
+constexpr int kPCLog = 14;
+constexpr uint32_t kPCBuckets = 1u << kPCLog;
+constexpr uint32_t kPCStash = 4096;
+constexpr uint32_t kPCStashMax = kPCStash / 2;
+constexpr int kPCMinBits = 32 - 15 - kPCLog;         // partition bits that leave a tag of at most 15
+constexpr uint64_t kCountRowsPerPartition = 15360;   // average build keys per partition (<= kPCBuckets with margin)
+constexpr int kPCRows = 16;                          // keys in flight per thread
+constexpr size_t kPCSmem = kPCBuckets * 8 + kPCStash * 4;
 
-__device__ __forceinline__ uint32_t pc_slot(int32_t key, int pbits) {
-  return (key_hash32(key) >> pbits) & (kPCCap - 1);
+// A zero 16-bit half in x.
+__device__ __forceinline__ bool pc_zero_half(uint32_t x, uint32_t y) {
+  return ((((x - 0x10001u) & ~x) | ((y - 0x10001u) & ~y)) & 0x80008000u) != 0u;
+}
+
+// f(key) for the keys [i0, i1) of a column, kPCRows of them loaded together per thread.
+template <class F>
+__device__ __forceinline__ void pc_each(const int32_t* __restrict__ col, uint32_t i0, uint32_t i1, F&& f) {
+  uint32_t i = i0 + threadIdx.x;
+  for (; i + (kPCRows - 1) * kPCThreads < i1; i += kPCRows * kPCThreads) {
+    int32_t k[kPCRows];
+#pragma unroll
+    for (int u = 0; u < kPCRows; u++) k[u] = __ldcs(col + i + u * kPCThreads);
+#pragma unroll
+    for (int u = 0; u < kPCRows; u++) f(k[u], i + u * kPCThreads);
+  }
+  // the last strip, its loads together too
+  int32_t k[kPCRows];
+#pragma unroll
+  for (int u = 0; u < kPCRows; u++) k[u] = i + u * kPCThreads < i1 ? __ldcs(col + i + u * kPCThreads) : kEmptyKey;
+#pragma unroll
+  for (int u = 0; u < kPCRows; u++)
+    if (i + u * kPCThreads < i1) f(k[u], i + u * kPCThreads);
 }
 
 __global__ void __launch_bounds__(kPCThreads, 1) partition_count_kernel(
     const int32_t* __restrict__ bk, const uint32_t* __restrict__ boff, const int32_t* __restrict__ pk,
     const uint32_t* __restrict__ poff, int pbits, uint8_t* flags, unsigned long long* count) {
-  extern __shared__ __align__(16) int32_t pc_key[];
-  const uint32_t part = blockIdx.x, mask = kPCCap - 1;
+  extern __shared__ __align__(16) unsigned char pc_smem[];
+  unsigned long long* bucket = reinterpret_cast<unsigned long long*>(pc_smem);
+  int32_t* stash = reinterpret_cast<int32_t*>(bucket + kPCBuckets);
+  __shared__ uint32_t stashed;
+  const uint32_t part = blockIdx.x;
   const uint32_t b0 = boff[part], b1 = boff[part + 1], p0 = poff[part], p1 = poff[part + 1];
-  const bool multi = (b1 - b0) > kPCChunk;
+  uint32_t chunk = kPCBuckets;
+  bool multi = (b1 - b0) > chunk;   // uniform, as every value a branch around a barrier tests
   uint32_t c = 0;
+  if (p0 == p1) return;
   if (multi)
     for (uint32_t i = p0 + threadIdx.x; i < p1; i += kPCThreads) flags[i] = 0;
-  for (uint32_t c0 = b0; c0 < b1; c0 += kPCChunk) {
-    const uint32_t c1 = min(c0 + kPCChunk, b1);
-    for (uint32_t i = threadIdx.x; i < kPCCap / 4; i += kPCThreads)
-      reinterpret_cast<int4*>(pc_key)[i] = make_int4(kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey);
+  for (uint32_t c0 = b0; c0 < b1;) {
+    const uint32_t c1 = min(c0 + chunk, b1);
+    __syncthreads();   // the previous chunk's probes are done
+    for (uint32_t i = threadIdx.x; i < kPCBuckets / 2; i += kPCThreads)
+      reinterpret_cast<ulonglong2*>(bucket)[i] = make_ulonglong2(0ull, 0ull);
+    for (uint32_t i = threadIdx.x; i < kPCStash / 4; i += kPCThreads)
+      reinterpret_cast<int4*>(stash)[i] = make_int4(kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey);
+    if (threadIdx.x == 0) stashed = 0;
     __syncthreads();
-    // duplicates take their own slots; a chunk fills at most half the table
-    for (uint32_t i0 = c0 + threadIdx.x; i0 < c1; i0 += kPCRows * kPCThreads) {
-      int32_t k[kPCRows];
-#pragma unroll
-      for (int u = 0; u < kPCRows; u++) {
-        const uint32_t i = i0 + u * kPCThreads;
-        k[u] = i < c1 ? __ldcs(bk + i) : kEmptyKey;
-      }
-#pragma unroll
-      for (int u = 0; u < kPCRows; u++) {
-        if (k[u] == kEmptyKey) continue;   // (an INT32_MIN key marks an empty slot and never matches)
-        uint32_t s = pc_slot(k[u], pbits);
-        for (uint32_t t = 0; t < kPCCap; t++, s = (s + 1) & mask)
-          if (atomicCAS(&pc_key[s], kEmptyKey, k[u]) == kEmptyKey) break;
-      }
-    }
-    __syncthreads();
-    for (uint32_t i0 = p0 + threadIdx.x; i0 < p1; i0 += kPCRows * kPCThreads) {
-      int32_t k[kPCRows];
-#pragma unroll
-      for (int u = 0; u < kPCRows; u++) {
-        const uint32_t i = i0 + u * kPCThreads;
-        k[u] = i < p1 ? __ldcs(pk + i) : kEmptyKey;
-      }
-      // (probing the kPCRows keys in lockstep rounds was slower: a warp then runs as many
-      // rounds as the longest probe chain among its 512 keys)
-#pragma unroll
-      for (int u = 0; u < kPCRows; u++) {
-        bool hit = false;
-        if (k[u] != kEmptyKey)
-          for (uint32_t s = pc_slot(k[u], pbits), t = 0; t < kPCCap; t++, s = (s + 1) & mask) {
-            const int32_t h = pc_key[s];
-            if (h == k[u]) { hit = true; break; }
-            if (h == kEmptyKey) break;
+    pc_each(bk, c0, c1, [&](int32_t k, uint32_t) {
+      if (k == kEmptyKey) return;   // (an INT32_MIN key never matches)
+      const uint32_t r = key_hash32(k) >> pbits;
+      const uint32_t tag = (r >> kPCLog) + 1u, tt = tag * 0x10001u;
+      unsigned long long* b = bucket + (r & (kPCBuckets - 1));
+      unsigned long long w = *b;
+      while (!pc_zero_half((uint32_t)w ^ tt, (uint32_t)(w >> 32) ^ tt)) {   // not there yet
+        const int s = (79 - __clzll((long long)w)) & ~15;                   // places fill from the low end
+        if (s < 64) {
+          const unsigned long long prev = atomicCAS(b, w, w | ((unsigned long long)tag << s));
+          if (prev == w) return;
+          w = prev;
+          continue;
+        }
+        bool counted = false;
+        for (uint32_t x = key_slot(k, kPCStash - 1);; x = (x + 1) & (kPCStash - 1)) {
+          int32_t e = stash[x];
+          if (e == kEmptyKey) {
+            if (!counted && atomicAdd(&stashed, 1u) >= kPCStashMax) return;   // (the chunk is redone below)
+            counted = true;
+            e = atomicCAS(&stash[x], kEmptyKey, k);
           }
-        if (multi) { if (hit) flags[i0 + u * kPCThreads] = 1; }
-        else c += hit;
+          if (e == kEmptyKey || e == k) return;
+        }
       }
-    }
+    });
     __syncthreads();
+    const uint32_t ns = stashed;
+    if (ns > kPCStashMax) {   // the stash overflowed: smaller chunks from this one on
+      if (!multi)
+        for (uint32_t i = p0 + threadIdx.x; i < p1; i += kPCThreads) flags[i] = 0;
+      multi = true;
+      chunk = kPCStashMax;
+      continue;
+    }
+    auto found = [&](int32_t k) {
+      const uint32_t r = key_hash32(k) >> pbits;
+      const uint32_t tt = ((r >> kPCLog) + 1u) * 0x10001u;
+      const uint2 w = reinterpret_cast<const uint2*>(bucket)[r & (kPCBuckets - 1)];
+      bool hit = pc_zero_half(w.x ^ tt, w.y ^ tt);   // (INT32_MIN is in no table, so it has no hit)
+      if (!hit && w.y >= 0x10000u && ns) {   // a full bucket, and keys in the stash
+        for (uint32_t z = key_slot(k, kPCStash - 1);; z = (z + 1) & (kPCStash - 1)) {
+          const int32_t e = stash[z];
+          if (e == kEmptyKey) break;
+          if (e == k) { hit = true; break; }
+        }
+      }
+      return hit;
+    };
+    if (multi) pc_each(pk, p0, p1, [&](int32_t k, uint32_t i) { if (found(k)) flags[i] = 1; });
+    else pc_each(pk, p0, p1, [&](int32_t k, uint32_t) { c += found(k); });
+    c0 = c1;
   }
-  if (multi)
+  if (multi) {
+    __syncthreads();
     for (uint32_t i = p0 + threadIdx.x; i < p1; i += kPCThreads) c += flags[i];
+  }
   c = __reduce_add_sync(FULL_MASK, c);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
 }
@@ -204,16 +260,15 @@ int partition_both(Call& call, const int32_t* build, uint64_t nb, const int32_t*
 int radix_join_count(Call& call, const int32_t* build_keys, uint64_t n_build, const int32_t* probe_keys, uint64_t n_probe,
                      unsigned long long* count) {
   if (n_build == 0 || n_probe == 0) return GPUDB_OK;
-  const int bits = radix_bits_for(n_build, kCountRowsPerPartition);
+  const int bits = std::max(kPCMinBits, radix_bits_for(n_build, kCountRowsPerPartition));
   Sides s;
   int rc = partition_both(call, build_keys, n_build, probe_keys, n_probe, bits, false, &s);
   if (rc) return rc;
   void* flags = nullptr;
   rc = scratch(call.ctx(), "rjoin.flags", n_probe + 16, &flags);
   if (rc) return rc;
-  const size_t smem = kPCCap * sizeof(int32_t);
-  GPUDB_CUDA(call.ctx(), kernel_smem(call.ctx(), (const void*)partition_count_kernel, smem));
-  GPUDB_LAUNCH(call, partition_count_kernel, 1u << bits, kPCThreads, smem, (const int32_t*)s.bk, (const uint32_t*)s.boff,
+  GPUDB_CUDA(call.ctx(), kernel_smem(call.ctx(), (const void*)partition_count_kernel, kPCSmem));
+  GPUDB_LAUNCH(call, partition_count_kernel, 1u << bits, kPCThreads, kPCSmem, (const int32_t*)s.bk, (const uint32_t*)s.boff,
                (const int32_t*)s.pk, (const uint32_t*)s.poff, bits, (uint8_t*)flags, count);
   return GPUDB_OK;
 }

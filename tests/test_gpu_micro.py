@@ -296,3 +296,36 @@ def test_radix_join_count_in_two_passes(engine):
     finally:
         for x in (db, dp):
             engine.device_free(x)
+
+
+def _unhash(h):
+    """Inverse of the engine's key hash (h ^= h >> 16; h *= 0x45d9f3b; h ^= h >> 16)."""
+    h = np.asarray(h, dtype=np.uint64)
+    h = h ^ (h >> np.uint64(16))
+    h = (h * np.uint64(pow(0x45D9F3B, -1, 1 << 32))) & np.uint64(0xFFFFFFFF)
+    return (h ^ (h >> np.uint64(16))).astype(np.uint32).view(np.int32)
+
+
+@pytest.mark.parametrize("per_bucket,buckets,dup", [(4, 3000, 1), (5, 300, 1), (5, 300, 60), (6, 2000, 1), (20_000, 1, 1),
+                                                    (1, 40_000, 1), (7, 900, 9)])
+def test_radix_join_count_full_buckets(engine, orc, per_bucket, buckets, dup):
+    """Build keys made to share the buckets of the count kernel's table: buckets that just fit,
+    that spill to the stash, that overfill the stash (the chunk is redone in smaller ones), keys
+    that repeat, and INT32_MIN on both sides (never matches). Probe keys of the same buckets with
+    other tags, and of full buckets that hold no such key."""
+    tag, bkt = np.meshgrid(np.arange(per_bucket), np.arange(buckets))
+    h = (tag.ravel().astype(np.uint64) << np.uint64(17)) | ((bkt.ravel() % (1 << 14)).astype(np.uint64) << np.uint64(3))
+    h |= np.uint64(5) + ((bkt.ravel() // (1 << 14)) % 3).astype(np.uint64)
+    b = np.repeat(_unhash(h), dup)
+    rng = np.random.default_rng(per_bucket)
+    b = np.concatenate([rng.permutation(b), np.array([-2**31, 77], np.int32)])
+    other = _unhash(h ^ (np.uint64(1) << np.uint64(31)))
+    p = rng.permutation(np.concatenate([_unhash(h), other, rng.integers(-2**31, 2**31, 5000).astype(np.int32),
+                                        np.array([-2**31, 77, 78], np.int32)]))
+    want = int((np.isin(p, b) & (p != -2**31)).sum())
+    db, dp = engine.to_device(b), engine.to_device(p)
+    try:
+        assert engine.hash_join_count(db, len(b), dp, len(p), capi.JOIN_RADIX) == want
+    finally:
+        engine.device_free(db)
+        engine.device_free(dp)
