@@ -456,7 +456,9 @@ int gpudb_create(int device, gpudb_ctx** out) {
   gpudb_ctx* ctx = new gpudb_ctx();
   ctx->device = device;
   ctx->sm_count = prop.multiProcessorCount;
-  cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
+  size_t free_mem = 0;
+  cudaError_t e = cudaMemGetInfo(&free_mem, &ctx->total_mem);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming);

@@ -839,13 +839,7 @@ int q3_direct(Call& call, const gpudb_customer& cu, const gpudb_orders& od, cons
 // reference's choice between its direct map and its hash table, src/q3.cpp:246).
 bool q3_direct_fits(gpudb_ctx* ctx, const gpudb_orders& od) {
   if (od.key_max < 0) return false;
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return false;
-  }
-  (void)ctx;
-  return ((double)od.key_max + 1.0) * 4.0 <= 0.3 * (double)total_b;
+  return ((double)od.key_max + 1.0) * 4.0 <= 0.3 * (double)ctx->total_mem;
 }
 
 // Global-table Q3 (steps 1-6 above). Result payload: {u64 groups, u128 rows[k]}.

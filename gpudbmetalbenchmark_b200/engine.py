@@ -38,6 +38,9 @@ TABLE_COLS = {
 }
 
 
+Q9_GROUP = np.dtype([("nation", np.int32), ("year", np.int32), ("profit", np.int64)])   # gpudb_q9_group
+
+
 class Table:
     """Columns of one table in device memory (or pinned host memory) owned by the engine."""
 
@@ -407,7 +410,11 @@ class Engine:
                                            C.byref(ps.struct()), C.byref(od.struct()), C.byref(ls), C.byref(p),
                                            groups, capacity, C.byref(n),
                                            C.byref(timing) if timing is not None else None, None))
-        return [(g.nation, g.year, g.profit) for g in groups[:min(n.value, capacity)]], n.value
+        m = min(n.value, capacity)
+        if not m:
+            return [], n.value
+        a = np.frombuffer(groups, dtype=Q9_GROUP, count=m)   # columns at a time: 12 us for 175 groups, 82 field by field
+        return list(zip(a["nation"].tolist(), a["year"].tolist(), a["profit"].tolist())), n.value
 
     def select_lt(self, col_ptr, n, value, bits_ptr=None, rows_ptr=None, timing=None):
         cnt = C.c_uint64()
