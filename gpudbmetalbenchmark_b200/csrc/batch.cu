@@ -5,7 +5,8 @@
 // evaluated on the rows while they are in registers:
 //  - a quad of rows whose ship dates no request can accept skips its other columns;
 //  - Q6 requests (up to kMaxQ6 per pass) keep per-thread register sums;
-//  - Q1 requests (up to kMaxQ1 per pass) differ only in their ship_date cutoff, so the
+//  - Q1 requests (up to kMaxQ1 per pass; on aligned columns the Q1 scan kernel takes them two at
+//    a time instead, launch_q1_riders) differ only in their ship_date cutoff, so the
 //    cutoffs are sorted and a row falls in bucket j = number of cutoffs below its ship
 //    date; it counts for every request whose sorted position is >= j. Each thread keeps
 //    private shared-memory sums per (bucket, flag, status) (no atomics; shared memory
@@ -396,18 +397,17 @@ int run_scan_batch(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32
   }
   std::vector<ScanGroup> groups;
   std::vector<ScanTile> tiles6, tiles1, tiles11;   // Q6 passes, Q1 passes of two / of one Q1 request
-  // Few requests on one table run the single-request kernels (both at the copy peak)
-  // instead of shared passes, whose per-row work for several requests makes them
-  // instruction-bound: over 60M rows a Q1 pass takes about 0.45 ms (two Q1 requests, Q6
-  // requests riding along) and a Q6 pass about 0.3 ms, against 0.23 ms for the Q1 kernel and
-  // 0.14 ms for the Q6 kernel. So up to kSoloQ1 Q1 requests on the same columns, and up to
-  // kSoloQ6 Q6 requests of a table without a Q1 pass, run alone.
-  // One Q1 request with up to kRideQ6 Q6 requests on its table runs the Q1 kernel with the
-  // Q6 requests riding along (one read of the rows for all of them, at the Q1 kernel's speed).
+  // Q1 requests on aligned columns go two to a read of the rows (the Q1 kernel with two buckets
+  // of sums), up to kRideQ6 Q6 requests riding along on each read: 350 us for two of each over 60M
+  // rows, 682 us one by one.
+  // What is left runs the single-request kernels while it is little (both at the copy peak): up
+  // to kSoloQ1 Q1 requests on the same columns, and up to kSoloQ6 Q6 requests of a table
+  // without a Q1 pass; more share the passes above, whose per-row work for several requests
+  // makes them instruction-bound (over 60M rows a Q1 pass takes about 0.45 ms and a Q6 pass
+  // about 0.3 ms, against 0.23 ms for the Q1 kernel and 0.14 ms for the Q6 kernel).
   constexpr size_t kSoloQ1 = 2, kSoloQ6 = 3, kRideQ6 = 4;
   struct Riding {
-    uint32_t q1;
-    std::vector<uint32_t> q6;
+    std::vector<uint32_t> q1, q6;
     gpudb_lineitem view;
   };
   std::vector<Riding> riding;
@@ -419,13 +419,29 @@ int run_scan_batch(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32
       solo_scans.emplace_back(k, row_view(*reqs[ids[k]].li, std::get<4>(kv.first), std::get<5>(kv.first)));
       solo[k] = 1;
     };
-    if (mb.q1.size() == 1 && mb.q1.begin()->second.size() == 1 && !mb.q6.empty() && mb.q6.size() <= kRideQ6) {
-      const uint32_t k = mb.q1.begin()->second[0];
-      riding.push_back(Riding{k, mb.q6, row_view(*reqs[ids[k]].li, std::get<4>(kv.first), std::get<5>(kv.first))});
-      solo[k] = 1;
-      for (uint32_t j : mb.q6) solo[j] = 1;
-      mb.q1.clear();
-      mb.q6.clear();
+    for (auto it = mb.q1.begin(); it != mb.q1.end();) {
+      std::vector<uint32_t>& l = it->second;
+      const gpudb_lineitem view = row_view(*reqs[ids[l[0]]].li, std::get<4>(kv.first), std::get<5>(kv.first));
+      if (!q1_shared_ok(ctx, view)) {
+        ++it;
+        continue;
+      }
+      std::sort(l.begin(), l.end(),   // neighbours share a pass
+                [&](uint32_t a, uint32_t b) { return reqs[ids[a]].q1.ship_le < reqs[ids[b]].q1.ship_le; });
+      for (size_t i = 0; i < l.size(); i += 2) {
+        Riding rd;
+        rd.view = view;
+        rd.q1.assign(l.begin() + i, l.begin() + std::min(l.size(), i + 2));
+        const size_t passes = (l.size() - i + 1) / 2;
+        for (size_t r = std::min(kRideQ6, (mb.q6.size() + passes - 1) / passes); r; r--) {
+          rd.q6.push_back(mb.q6.back());
+          mb.q6.pop_back();
+        }
+        for (uint32_t k : rd.q1) solo[k] = 1;
+        for (uint32_t k : rd.q6) solo[k] = 1;
+        riding.push_back(rd);
+      }
+      it = mb.q1.erase(it);
     }
     for (auto it = mb.q1.begin(); it != mb.q1.end();) {
       if (it->second.size() <= kSoloQ1) {
@@ -522,14 +538,20 @@ int run_scan_batch(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32
     if (rc) return rc;
   }
   for (const Riding& rd : riding) {
+    std::vector<gpudb_q1_params> p1;
     std::vector<gpudb_q6_params> p6;
-    std::vector<void*> o6;
+    std::vector<void*> o1, o6;
+    std::vector<uint32_t*> s1;
+    for (uint32_t j : rd.q1) {
+      p1.push_back(reqs[ids[j]].q1);
+      o1.push_back(dres + status_bytes + (size_t)offs[j] * 8);
+      s1.push_back(reinterpret_cast<uint32_t*>(dres) + j);
+    }
     for (uint32_t j : rd.q6) {
       p6.push_back(reqs[ids[j]].q6);
       o6.push_back(dres + status_bytes + (size_t)offs[j] * 8);
     }
-    rc = launch_q1_riders(call, rd.view, reqs[ids[rd.q1]].q1, dres + status_bytes + (size_t)offs[rd.q1] * 8,
-                          reinterpret_cast<uint32_t*>(dres) + rd.q1, (int)p6.size(), p6.data(), o6.data());
+    rc = launch_q1_riders(call, rd.view, (int)p1.size(), p1.data(), o1.data(), s1.data(), (int)p6.size(), p6.data(), o6.data());
     if (rc) return rc;
   }
   for (const auto& sq : solo_scans) {

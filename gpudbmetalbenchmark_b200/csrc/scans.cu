@@ -250,7 +250,7 @@ __device__ __forceinline__ void q1_fold(Q1Acc& a, u128* partials, unsigned* tick
 // word cannot overflow before 2^32 blocks, and the add needs no return value (no round trip,
 // unlike a carry-propagating 128-bit add). The value is sum_j word_j * 2^32j, exact.
 constexpr int kQ1AccCopies = 16;
-constexpr size_t kQ1GaccWords = (size_t)kQ1AccCopies * 6 * kQ1Raw * 3;
+constexpr size_t kQ1GaccWords = (size_t)kQ1AccCopies * 2 * 6 * kQ1Raw * 3;   // (two requests' worth)
 
 __device__ __forceinline__ void red_add_limbs(unsigned long long* w, u128 v) {
   const unsigned long long l0 = (unsigned long long)v & 0xFFFFFFFFull;
@@ -266,17 +266,27 @@ __device__ __forceinline__ void red_add_limbs(unsigned long long* w, u128 v) {
 // quantity and discount sum) and adds the block's totals into its copy of the limb words of
 // `gacc` (kQ1GaccWords); the last block turns them into the output and zeroes `gacc` for the
 // next launch (it is zero when first allocated). No per-block partials are read back.
-template <int T>
-__device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, unsigned long long* gacc, unsigned* ticket, u128* out,
-                                             uint32_t* status, uint32_t* hstatus) {
+// NQ1 = 2: the sums come in two buckets of 24 columns (rows up to the first request's cutoff, rows
+// between the cutoffs), `bad` in bit j for bucket j; the second request's totals are both.
+struct Q1Requests {
+  int32_t cut[2];          // ship_date cutoffs, ascending
+  u128* out[2];
+  uint32_t* status[2];
+};
+
+template <int T, int NQ1>
+__device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, unsigned long long* gacc, unsigned* ticket,
+                                             const Q1Requests& rq, uint32_t* hstatus) {
   constexpr int W = T / 32;
   static_assert(24 % W == 0, "whole columns per warp");
-  __shared__ u128 tot[6 * kQ1Raw];
+  __shared__ u128 tot[NQ1 * 6 * kQ1Raw];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // also orders every thread's shared-memory sums before the column reads
-  if (__syncthreads_or(bad) && threadIdx.x == 0) set_status(status, ST_DOMAIN);
-  for (int c = warp; c < 24; c += W) {
-    const int metric = c / 6, g = c % 6;
+#pragma unroll
+  for (int j = 0; j < NQ1; j++)
+    if (__syncthreads_or(bad & ((2u << j) - 1u)) && threadIdx.x == 0) set_status(rq.status[j], ST_DOMAIN);
+  for (int c = warp; c < NQ1 * 24; c += W) {
+    const int metric = c % 24 / 6, g = c / 24 * 6 + c % 6;   // g: bucket and group
     u128 s0 = 0, s1 = 0, s2 = 0;
 #pragma unroll 4
     for (int i = lane; i < T; i += 32) {
@@ -296,7 +306,7 @@ __device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, 
     }
     if (lane == 0) {
       // raw metrics: count, qty, E, ED, EDT, dsum
-      unsigned long long* o = gacc + ((size_t)(blockIdx.x % kQ1AccCopies) * 6 * kQ1Raw + g * kQ1Raw) * 3;
+      unsigned long long* o = gacc + ((size_t)(blockIdx.x % kQ1AccCopies) * NQ1 * 6 * kQ1Raw + g * kQ1Raw) * 3;
       if (metric == 0) {
         red_add_limbs(o + 0 * 3, s0);
         red_add_limbs(o + 1 * 3, s1);
@@ -307,11 +317,11 @@ __device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, 
     }
   }
   if (!grid_last_block(ticket)) return;
-  if (threadIdx.x < 6 * kQ1Raw) {
+  if (threadIdx.x < NQ1 * 6 * kQ1Raw) {
     u128 v = 0;
 #pragma unroll
     for (int c = 0; c < kQ1AccCopies; c++) {
-      unsigned long long* w = gacc + ((size_t)c * 6 * kQ1Raw + threadIdx.x) * 3;
+      unsigned long long* w = gacc + ((size_t)c * NQ1 * 6 * kQ1Raw + threadIdx.x) * 3;
       v += (u128)__ldcg(w) + ((u128)__ldcg(w + 1) << 32) + ((u128)__ldcg(w + 2) << 64);
       w[0] = 0;
       w[1] = 0;
@@ -320,12 +330,17 @@ __device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, 
     tot[threadIdx.x] = v;
   }
   __syncthreads();
-  if (threadIdx.x < 6) {
-    const int g = threadIdx.x;
-    const u128* r = tot + g * kQ1Raw;
+  if (threadIdx.x < NQ1 * 6) {
+    const int j = NQ1 > 1 ? threadIdx.x / 6 : 0, g = threadIdx.x - 6 * j;
+    u128 r[kQ1Raw];
+#pragma unroll
+    for (int m = 0; m < kQ1Raw; m++) {
+      r[m] = tot[g * kQ1Raw + m];
+      if (NQ1 > 1 && j) r[m] += tot[(6 + g) * kQ1Raw + m];
+    }
     const u128 disc_price = (u128)100 * r[2] - r[3];
     const u128 charge = (u128)100 * disc_price + r[4];
-    u128* o = out + g * kQ1Metrics;
+    u128* o = rq.out[j] + g * kQ1Metrics;
     if (hstatus) {   // one launch, the host slot: overwrite
       o[0] = r[0];
       o[1] = r[1];
@@ -345,8 +360,8 @@ __device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, 
   // the host slot takes the status every block has OR-ed in (visible past the ticket), and
   // the launch's own status word is left at zero for the next launch
   if (hstatus && threadIdx.x == 0) {
-    *hstatus = __ldcg(status);
-    *status = 0u;
+    *hstatus = __ldcg(rq.status[0]);
+    *rq.status[0] = 0u;
   }
 }
 
@@ -679,7 +694,7 @@ __global__ void __launch_bounds__(THREADS, 1) q1_ring_smem_kernel(const int32_t*
 // 128-bit loads straight from HBM with the accumulators in shared memory: registers stay low
 // (several blocks per SM), and each thread keeps two quads (208 bytes) of loads in flight.
 constexpr int kQ1SmemThreads = 256;
-constexpr size_t kQ1AccBytes = (size_t)4 * 6 * kQ1SmemThreads * 8;   // 49,152
+constexpr size_t kQ1AccBytes = (size_t)4 * 6 * kQ1SmemThreads * 8;   // 49,152 per Q1 request
 
 // Q6 requests evaluated on the rows a Q1 scan reads (one read of the table for both): their
 // constants, and the two words (revenue, rows matched) each one adds into.
@@ -693,36 +708,41 @@ struct Q6Riders {
 // more loads in flight for tables that end in one short wave). NQ6: Q6 requests riding along
 // (register sums per request, added into their words at the end). QPI: 16-byte quads per
 // thread per step (2 by default; 4: variant 9; 1 with four blocks per SM: variant 10).
-template <int MINB, int NQ6, int QPI = 2>
+// NQ1 = 2: two requests in one read of the rows. Their cutoffs split the rows into two buckets of
+// sums (96 KB a block, still two blocks per SM), so a row costs what it costs for one request. 60M
+// rows, two Q1 and two Q6 requests: 350 us, against 682 us for their four kernels (226 us each
+// Q1, 109 and 122 us the Q6).
+template <int MINB, int NQ6, int QPI = 2, int NQ1 = 1>
 __global__ void __launch_bounds__(kQ1SmemThreads, MINB) q1_vec_smem_kernel(const int4* __restrict__ ship4, const int4* __restrict__ qty4,
                                                                      const longlong2* __restrict__ ext2, const int4* __restrict__ disc4,
                                                                      const int4* __restrict__ tax4, const uint32_t* __restrict__ flag4,
-                                                                     const uint32_t* __restrict__ stat4, uint64_t n, int32_t ship_le,
-                                                                     unsigned long long* gacc, unsigned* ticket, u128* out, uint32_t* status,
+                                                                     const uint32_t* __restrict__ stat4, uint64_t n, Q1Requests rq,
+                                                                     unsigned long long* gacc, unsigned* ticket,
                                                                      uint32_t* hstatus, Q6Riders riders) {
   constexpr int T = kQ1SmemThreads;
-  extern __shared__ __align__(16) uint64_t q1_acc[];   // [4 metrics][6 groups][T]
+  extern __shared__ __align__(16) uint64_t q1_acc[];   // [NQ1 buckets][4 metrics][6 groups][T]
   const int t = threadIdx.x;
 #pragma unroll
-  for (int i = 0; i < 24; i++) q1_acc[i * T + t] = 0;
+  for (int i = 0; i < NQ1 * 24; i++) q1_acc[i * T + t] = 0;
   uint32_t bad = 0;
   int64_t rrev[NQ6 > 0 ? NQ6 : 1];
-  uint64_t rcnt[NQ6 > 0 ? NQ6 : 1];
+  uint32_t rcnt[NQ6 > 0 ? NQ6 : 1];
 #pragma unroll
   for (int r = 0; r < NQ6; r++) { rrev[r] = 0; rcnt[r] = 0; }
   auto row = [&](int32_t s, int32_t qt, int64_t e, int32_t d, int32_t tx, uint32_t f, uint32_t st) {
+    const uint64_t ed = (uint64_t)(e * (int64_t)d);
 #pragma unroll
     for (int r = 0; r < NQ6; r++) {
       const bool m = q6_pass(s, d, qt, riders.p[r]);
-      rrev[r] += m ? e * (int64_t)d : 0;
+      rrev[r] += m ? (int64_t)ed : 0;
       rcnt[r] += m;
     }
-    if (!((s <= ship_le) & (f <= 2u) & (st <= 1u))) return;
-    bad |= ((uint32_t)qt >= 65536u) | ((uint32_t)d > 100u) | ((uint32_t)tx > 100u) | ((uint64_t)e >= (1ull << 36));
-    const uint64_t ed = (uint64_t)e * (uint32_t)d;
+    if (!((s <= rq.cut[NQ1 - 1]) & (f <= 2u) & (st <= 1u))) return;
+    const uint32_t bucket = NQ1 > 1 && s > rq.cut[0] ? 1u : 0u;
+    bad |= (uint32_t)(((uint32_t)qt >= 65536u) | ((uint32_t)d > 100u) | ((uint32_t)tx > 100u) | ((uint64_t)e >= (1ull << 36))) << bucket;
     const uint64_t edt = ((uint64_t)e * 100u - ed) * (uint32_t)tx;
     const uint64_t pk = ((uint64_t)(uint32_t)qt << 32) | ((uint64_t)(uint32_t)d << 13) | 1u;
-    uint64_t* p = q1_acc + (f * 2u + st) * T + t;
+    uint64_t* p = q1_acc + (bucket * 24u + f * 2u + st) * T + t;
     p[0] += pk;
     p[6 * T] += (uint64_t)e;
     p[12 * T] += ed;
@@ -776,7 +796,7 @@ __global__ void __launch_bounds__(kQ1SmemThreads, MINB) q1_vec_smem_kernel(const
       if (c) atomicAdd(riders.out[r] + 1, c);
     }
   }
-  q1_smem_fold<T>(q1_acc, bad, gacc, ticket, out, status, hstatus);
+  q1_smem_fold<T, NQ1>(q1_acc, bad, gacc, ticket, rq, hstatus);
 }
 
 bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
@@ -845,12 +865,11 @@ int launch_q6(Call& call, const gpudb_lineitem& c, const gpudb_q6_params& p, voi
 // launch's status word is the one in the scratch header beside the ticket, which the last
 // block copies to the host slot and leaves at zero.
 using Q1SmemKernel = void (*)(const int4*, const int4*, const longlong2*, const int4*, const int4*, const uint32_t*,
-                              const uint32_t*, uint64_t, int32_t, unsigned long long*, unsigned*, u128*, uint32_t*,
-                              uint32_t*, Q6Riders);
-static int launch_q1_smem(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, void* out, uint32_t* status,
-                          Q1SmemKernel kern, const Q6Riders& riders, uint32_t* hstatus = nullptr) {
+                              const uint32_t*, uint64_t, Q1Requests, unsigned long long*, unsigned*, uint32_t*, Q6Riders);
+static int launch_q1_smem(Call& call, const gpudb_lineitem& c, Q1Requests rq, int nq1, Q1SmemKernel kern,
+                          const Q6Riders& riders, uint32_t* hstatus = nullptr) {
   gpudb_ctx* ctx = call.ctx();
-  const size_t smem = kQ1AccBytes;
+  const size_t smem = kQ1AccBytes * nq1;
   GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)kern, smem));
   const int per_sm = kernel_occupancy(ctx, (const void*)kern, kQ1SmemThreads, smem);
   const uint64_t min_blocks = (c.n_rows + (uint64_t)kQ1SmemThreads * kQ1RowsPerThread - 1) /
@@ -863,12 +882,10 @@ static int launch_q1_smem(Call& call, const gpudb_lineitem& c, const gpudb_q1_pa
   unsigned* ticket = nullptr;
   int rc = scan_scratch(ctx, "q1.acc", kQ1GaccWords * sizeof(unsigned long long), &part, &ticket);
   if (rc) return rc;
-  if (hstatus) status = ticket + 1;
+  if (hstatus) rq.status[0] = ticket + 1;
   GPUDB_LAUNCH(call, kern, grid, kQ1SmemThreads, smem, (const int4*)c.ship_date, (const int4*)c.quantity,
                (const longlong2*)c.ext_price, (const int4*)c.discount, (const int4*)c.tax, (const uint32_t*)c.flag,
-               (const uint32_t*)c.status, c.n_rows, p.ship_le, (unsigned long long*)part, ticket, (u128*)out, status,
-               hstatus,
-               riders);
+               (const uint32_t*)c.status, c.n_rows, rq, (unsigned long long*)part, ticket, hstatus, riders);
   return GPUDB_OK;
 }
 
@@ -886,6 +903,10 @@ static int q1_variant(const gpudb_ctx* ctx, const gpudb_lineitem& c) {
   return variant;
 }
 
+static Q1Requests q1_one(const gpudb_q1_params& p, void* out, uint32_t* status) {
+  return Q1Requests{{p.ship_le, 0}, {static_cast<u128*>(out), nullptr}, {status, nullptr}};
+}
+
 static Q1SmemKernel q1_smem_kernel(int variant) {
   return variant == 8  ? q1_vec_smem_kernel<3, 0, 2>
        : variant == 9  ? q1_vec_smem_kernel<2, 0, 4>
@@ -900,7 +921,7 @@ int launch_q1(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, voi
   // 0 auto, 1 TMA 2048-row tiles x 4 stages, 2 vector loads, 3 one row per thread,
   // 4 TMA 4096-row tiles x 2 stages, 5/6 TMA rings, 7-10 shared-memory sums
   const int variant = q1_variant(ctx, c);
-  if (variant >= 7 && variant <= 10) return launch_q1_smem(call, c, p, out, status, q1_smem_kernel(variant), Q6Riders{});
+  if (variant >= 7 && variant <= 10) return launch_q1_smem(call, c, q1_one(p, out, status), 1, q1_smem_kernel(variant), Q6Riders{});
   if (variant == 1 || variant >= 4) {
     const uint32_t R = (variant == 1 || variant == 5) ? 2048u : variant == 6 ? 1024u : 4096u;
     const int threads = variant == 6 ? 256 : kQ1TmaThreads;
@@ -945,12 +966,16 @@ int launch_q1(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, voi
   return GPUDB_OK;
 }
 
-int launch_q1_riders(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, void* out, uint32_t* status,
-                     int n6, const gpudb_q6_params* q6, void* const* q6out) {
-  const bool vec = aligned(c.ship_date, 16) && aligned(c.quantity, 16) && aligned(c.ext_price, 16) &&
-                   aligned(c.discount, 16) && aligned(c.tax, 16) && aligned(c.flag, 4) && aligned(c.status, 4);
-  if (n6 <= 0 || n6 > kMaxRiders || !vec || c.n_rows == 0 || call.ctx()->scan_variant != 0) {
-    int rc = launch_q1(call, c, p, out, status);   // one kernel per request
+bool q1_shared_ok(const gpudb_ctx* ctx, const gpudb_lineitem& c) {
+  return aligned(c.ship_date, 16) && aligned(c.quantity, 16) && aligned(c.ext_price, 16) && aligned(c.discount, 16) &&
+         aligned(c.tax, 16) && aligned(c.flag, 4) && aligned(c.status, 4) && c.n_rows > 0 && ctx->scan_variant == 0;
+}
+
+int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1_params* q1, void* const* q1out,
+                     uint32_t* const* q1status, int n6, const gpudb_q6_params* q6, void* const* q6out) {
+  if (n1 < 1 || n1 > 2 || n6 < 0 || n6 > kMaxRiders || !q1_shared_ok(call.ctx(), c)) {
+    int rc = GPUDB_OK;   // one kernel per request
+    for (int r = 0; !rc && r < n1; r++) rc = launch_q1(call, c, q1[r], q1out[r], q1status[r]);
     for (int r = 0; !rc && r < n6; r++) rc = launch_q6(call, c, q6[r], q6out[r]);
     return rc;
   }
@@ -959,9 +984,22 @@ int launch_q1_riders(Call& call, const gpudb_lineitem& c, const gpudb_q1_params&
     rd.p[r] = Q6P{q6[r].ship_lo, q6[r].ship_hi, q6[r].disc_lo, q6[r].disc_hi, q6[r].qty_lt};
     rd.out[r] = static_cast<unsigned long long*>(q6out[r]);
   }
-  static constexpr Q1SmemKernel kRiding[kMaxRiders] = {q1_vec_smem_kernel<2, 1>, q1_vec_smem_kernel<2, 2>,
-                                                       q1_vec_smem_kernel<2, 3>, q1_vec_smem_kernel<2, 4>};
-  return launch_q1_smem(call, c, p, out, status, kRiding[n6 - 1], rd);
+  Q1Requests rq = q1_one(q1[0], q1out[0], q1status[0]);
+  if (n1 == 2) {
+    const int lo = q1[1].ship_le < q1[0].ship_le ? 1 : 0;
+    for (int j = 0; j < 2; j++) {
+      const int r = j ? 1 - lo : lo;
+      rq.cut[j] = q1[r].ship_le;
+      rq.out[j] = static_cast<u128*>(q1out[r]);
+      rq.status[j] = q1status[r];
+    }
+  }
+  static constexpr Q1SmemKernel kRiding[2][kMaxRiders + 1] = {
+      {q1_vec_smem_kernel<2, 0>, q1_vec_smem_kernel<2, 1>, q1_vec_smem_kernel<2, 2>, q1_vec_smem_kernel<2, 3>,
+       q1_vec_smem_kernel<2, 4>},
+      {q1_vec_smem_kernel<2, 0, 2, 2>, q1_vec_smem_kernel<2, 1, 2, 2>, q1_vec_smem_kernel<2, 2, 2, 2>,
+       q1_vec_smem_kernel<2, 3, 2, 2>, q1_vec_smem_kernel<2, 4, 2, 2>}};
+  return launch_q1_smem(call, c, rq, n1, kRiding[n1 - 1][n6], rd);
 }
 
 }  // namespace gpudb
@@ -1011,7 +1049,7 @@ extern "C" int gpudb_q1_group6(gpudb_ctx* ctx, const gpudb_lineitem* li, const g
   if ((rc = direct ? call.begin_direct(bytes) : call.begin(bytes))) return rc;
   const gpudb_q1_params pp = *p;
   if (uint8_t* d = call.direct_slot()) {
-    rc = launch_q1_smem(call, *li, pp, d + kSlotHeader, nullptr, q1_smem_kernel(variant), Q6Riders{},
+    rc = launch_q1_smem(call, *li, q1_one(pp, d + kSlotHeader, nullptr), 1, q1_smem_kernel(variant), Q6Riders{},
                         reinterpret_cast<uint32_t*>(d));
   } else {
     void* dout = call.result<void>();

@@ -14,12 +14,15 @@ constexpr size_t kQ1ResultBytes = 6 * 6 * 16;      // 6 groups x {count, qty, ba
 // overwrites `out` in that slot instead: one launch over the whole table.
 int launch_q6(Call& call, const gpudb_lineitem& c, const gpudb_q6_params& p, void* out, uint32_t* hstatus = nullptr);
 int launch_q1(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, void* out, uint32_t* status = nullptr);
-// One Q1 scan that also evaluates up to 4 Q6 requests on the rows it reads (one read of the
-// table for all of them); each Q6 request adds into its own kQ6ResultBytes words. Falls back
-// to one kernel per request for columns off 16 bytes, more Q6 requests, or a Q1 kernel
-// variant chosen on the context.
-int launch_q1_riders(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, void* out, uint32_t* status,
-                     int n6, const gpudb_q6_params* q6, void* const* q6out);
+// One scan for n1 (1 or 2) Q1 requests that also evaluates up to 4 Q6 requests on the rows it reads
+// (one read of the table for all of them); each request adds into its own words and, Q1,
+// reports into its own status word. Falls back to one kernel per request for columns off 16
+// bytes, more requests, or a Q1 kernel variant chosen on the context.
+int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1_params* q1, void* const* q1out,
+                     uint32_t* const* q1status, int n6, const gpudb_q6_params* q6, void* const* q6out);
+
+// Whether launch_q1_riders would share one read of these columns between requests.
+bool q1_shared_ok(const gpudb_ctx* ctx, const gpudb_lineitem& c);
 
 // Host result from the kQ1ResultBytes device words of one Q1 scan.
 void q1_result_from(const uint8_t* words, gpudb_q1_result* out);

@@ -277,3 +277,29 @@ def test_heavy_lane_takes_the_large_scans(engine):
     assert st["completed"] == len(jobs) and st["failed"] == 0
     with pytest.raises(capi.GpudbError):
         Server(lanes=2, heavy_lanes=2)
+
+
+@pytest.mark.parametrize("cuts", [(500, 1500), (1500, 500), (900, 900), (-1, 1200), (2**31 - 1, 700), (1000, 1400, 1800)])
+def test_two_q1_requests_in_one_scan(engine, orc, cuts):
+    """Q1 requests that share a scan: cutoffs in either order, equal, selecting nothing and
+    everything; and a value outside the exact-arithmetic domain above the lower cutoffs fails
+    only the requests that read its row."""
+    n = 50_003
+    for bad_day in (None, 1300):
+        li = orc.lineitem(n, seed=91)
+        if bad_day is not None:
+            li["ship_date"][7] = bad_day
+            li["discount"][7] = 101
+        t = engine.upload("lineitem", li)
+        s = t.lineitem()
+        reqs = (capi.Request * len(cuts))()
+        outs = [capi.Q1Result() for _ in cuts]
+        for r, c, o in zip(reqs, cuts, outs):
+            r.pipeline, r.li, r.q1, r.q1_out = capi.PIPE_Q1, C.pointer(s), capi.Q1Params(c, 0), C.pointer(o)
+        engine._check(engine.lib.gpudb_batch_run(engine.ctx, reqs, len(cuts), None, None))
+        for r, c, o in zip(reqs, cuts, outs):
+            if bad_day is not None and c >= bad_day:
+                assert r.status == capi.E_INVALID
+            else:
+                assert r.status == capi.OK and q1_to_dict(o) == orc.q1(li, c), c
+        engine.free(t)
