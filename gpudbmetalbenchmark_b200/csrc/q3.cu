@@ -15,7 +15,8 @@
 //  4. orders_insert_kernel: atomicCAS insertion; each slot is {key, date, revenue} and a
 //     parallel hit counter, so the orders table doubles as the per-order aggregation table
 //     (the group key equals the join key).
-//  5. q3_probe_kernel: one lane per fact row; runs of equal order keys (adjacent rows of one
+//  5. q3_quad_kernel (aligned columns; the same steps on quads of rows, see there) or
+//     q3_probe_kernel: one lane per fact row; runs of equal order keys (adjacent rows of one
 //     order) are found with a warp ballot, only the run head probes the table (after a test
 //     of the order-key bitmap that step 4 sets, which turns away most misses), and each row
 //     that joins adds its revenue and a count with one atomic each (a few percent of rows).
@@ -382,21 +383,33 @@ __global__ void __launch_bounds__(256) q3_direct_probe_kernel(
   }
 }
 
-// Quad form of the direct probe, for 16-byte aligned columns: a lane takes kDirectQuads quads
+// Quad form of the probes, for 16-byte aligned columns: a lane takes kDirectQuads quads
 // (4 consecutive rows each: one 16-byte load of keys and one of ship dates per quad). Inside a
 // quad, rows of one order are adjacent, so the lane looks up each distinct key among its
 // passing rows once (bitmap word, then slot), and rows of equal slot are summed before one
 // atomic pair. ext_price / discount of a quad load only when one of its rows joins. The
 // kDirectQuads quads' loads are issued phase by phase, all in flight together. Tail rows past
 // the last whole quad go one per thread.
+// DIRECT: the slot comes from the direct map `omap`, and block 0 seals the dense slots. Else it
+// comes from the hash table of *cap_p slots: every key's home slot is read in one phase, and
+// only a key that finds another key there walks on; `okbm` (null, or off when *okbm_off is set)
+// turns most misses away first. 6M rows: 48 us with 32-row batches and a walk per run, 31 us
+// here; whole call in global mode, 60M rows: 575 -> 437 us, 6M: 136 -> 121 us.
+// (Loading the next step's quads ahead took 231 us of 60M rows instead of 212: the registers
+// cost a block per SM. So did prefetching them into L2.)
 constexpr int kDirectQuads = 2;
 
-__global__ void __launch_bounds__(256) q3_direct_quad_kernel(
+template <bool DIRECT>
+__global__ void __launch_bounds__(256) q3_quad_kernel(
     const int4* __restrict__ lkey4, const int4* __restrict__ lship4, const longlong2* __restrict__ lext2,
     const int4* __restrict__ ldisc4, uint64_t n, int32_t ship_gt, const uint32_t* __restrict__ okbm,
     const int32_t* __restrict__ omap, int32_t key_max, Q3Slot* ht, uint32_t* hits, const uint32_t* count,
-    uint32_t* cap_out) {
-  if (blockIdx.x == 0) seal_dense_slots(count, hits, cap_out);
+    uint32_t* cap_out, const uint32_t* cap_p, const uint32_t* okbm_off) {
+  if (DIRECT && blockIdx.x == 0) seal_dense_slots(count, hits, cap_out);
+  const uint32_t cap = DIRECT ? 0u : *cap_p;
+  if (!DIRECT && okbm && *okbm_off != 0u) okbm = nullptr;
+  // keys that can have a slot
+  const int32_t lo = DIRECT || okbm ? 0 : INT32_MIN + 1, hi = DIRECT || okbm ? key_max : INT32_MAX;
   constexpr int U = kDirectQuads;
   const uint64_t nq = n >> 2;
   const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
@@ -420,18 +433,30 @@ __global__ void __launch_bounds__(256) q3_direct_quad_kernel(
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int r = 4 * u + i;
-        const bool p = ship[r] > ship_gt && key[r] >= 0 && key[r] <= key_max;
+        const bool p = ship[r] > ship_gt && key[r] >= lo && key[r] <= hi;
         pass |= (uint32_t)p << r;
         if (p && key[r] != last) { want |= 1u << r; last = key[r]; }
       }
     }
     uint32_t word[4 * U];
 #pragma unroll
-    for (int r = 0; r < 4 * U; r++) word[r] = (want >> r & 1u) ? __ldg(okbm + ((uint32_t)key[r] >> 5)) : 0u;
-    int32_t slot[4 * U];
-#pragma unroll
     for (int r = 0; r < 4 * U; r++)
-      slot[r] = ((want >> r & 1u) && (word[r] >> ((uint32_t)key[r] & 31u) & 1u)) ? __ldg(omap + key[r]) : -1;
+      word[r] = (want >> r & 1u) ? (DIRECT || okbm ? __ldg(okbm + ((uint32_t)key[r] >> 5)) >> ((uint32_t)key[r] & 31u) : 1u) : 0u;
+    int32_t slot[4 * U];
+    if (DIRECT) {
+#pragma unroll
+      for (int r = 0; r < 4 * U; r++) slot[r] = (word[r] & 1u) ? __ldg(omap + key[r]) : -1;
+    } else {
+      int32_t home[4 * U];
+#pragma unroll
+      for (int r = 0; r < 4 * U; r++) {
+        slot[r] = (word[r] & 1u) ? (int32_t)key_slot(key[r], cap - 1) : -1;
+        home[r] = slot[r] >= 0 ? __ldg(&ht[slot[r]].key) : 0;
+      }
+#pragma unroll
+      for (int r = 0; r < 4 * U; r++)
+        if (slot[r] >= 0 && home[r] != key[r]) slot[r] = home[r] == kEmptyKey ? -1 : ht_find(ht, cap, key[r]);
+    }
     // rows that did not look up take the slot of the previous row of the quad (same key)
 #pragma unroll
     for (int u = 0; u < U; u++)
@@ -482,12 +507,14 @@ __global__ void __launch_bounds__(256) q3_direct_quad_kernel(
     const int32_t* k1 = reinterpret_cast<const int32_t*>(lkey4);
     const int32_t* s1 = reinterpret_cast<const int32_t*>(lship4);
     const int32_t k = k1[r];
-    if (s1[r] > ship_gt && k >= 0 && k <= key_max && bitmap_test(okbm, k)) {
-      const int32_t sl = omap[k];
-      const int64_t e = reinterpret_cast<const int64_t*>(lext2)[r];
-      const int32_t dd = reinterpret_cast<const int32_t*>(ldisc4)[r];
-      atomicAdd(&ht[sl].rev, (unsigned long long)(e * (int64_t)(100 - dd)));
-      atomicAdd(&hits[sl], 1u);
+    if (s1[r] > ship_gt && k >= lo && k <= hi && (!(DIRECT || okbm) || bitmap_test(okbm, k))) {
+      const int32_t sl = DIRECT ? omap[k] : ht_find(ht, cap, k);
+      if (sl >= 0) {
+        const int64_t e = reinterpret_cast<const int64_t*>(lext2)[r];
+        const int32_t dd = reinterpret_cast<const int32_t*>(ldisc4)[r];
+        atomicAdd(&ht[sl].rev, (unsigned long long)(e * (int64_t)(100 - dd)));
+        atomicAdd(&hits[sl], 1u);
+      }
     }
   }
 }
@@ -807,11 +834,11 @@ int q3_direct(Call& call, const gpudb_customer& cu, const gpudb_orders& od, cons
       const uint64_t per_block = 256 * 4 * kDirectQuads;
       const unsigned g = (unsigned)std::max<uint64_t>(
           1, std::min<uint64_t>((c.n_rows + per_block - 1) / per_block,
-                                (uint64_t)sms * kernel_occupancy(ctx, (const void*)q3_direct_quad_kernel, 256, 0)));
-      GPUDB_LAUNCH(call, q3_direct_quad_kernel, g, 256, 0, (const int4*)c.order_key, (const int4*)c.ship_date,
+                                (uint64_t)sms * kernel_occupancy(ctx, (const void*)q3_quad_kernel<true>, 256, 0)));
+      GPUDB_LAUNCH(call, q3_quad_kernel<true>, g, 256, 0, (const int4*)c.order_key, (const int4*)c.ship_date,
                    (const longlong2*)c.ext_price, (const int4*)c.discount, c.n_rows, p.ship_date_gt,
                    (const uint32_t*)okbm, (const int32_t*)omap, key_max, (Q3Slot*)ht, (uint32_t*)hits,
-                   (const uint32_t*)cnt, cnt + 1);
+                   (const uint32_t*)cnt, cnt + 1, (const uint32_t*)nullptr, (const uint32_t*)nullptr);
     } else {
       const uint64_t per_block = 256 * kDirectBatches;
       const unsigned g = (unsigned)std::max<uint64_t>(
@@ -888,6 +915,18 @@ int q3_global(Call& call, const gpudb_customer& cu, const gpudb_orders& od, cons
   const uint32_t mask = LI_ORDER | LI_SHIP | LI_EXT | LI_DISC;
   rc = stream_lineitem(call, li, mask, 0, [&](const gpudb_lineitem& c) {
     if (c.n_rows == 0) return (int)GPUDB_OK;
+    auto a16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    if (a16(c.order_key) && a16(c.ship_date) && a16(c.ext_price) && a16(c.discount)) {
+      const uint64_t per_block = 256 * 4 * kDirectQuads;
+      const unsigned gq = (unsigned)std::max<uint64_t>(
+          1, std::min<uint64_t>((c.n_rows + per_block - 1) / per_block,
+                                (uint64_t)sms * kernel_occupancy(ctx, (const void*)q3_quad_kernel<false>, 256, 0)));
+      GPUDB_LAUNCH(call, q3_quad_kernel<false>, gq, 256, 0, (const int4*)c.order_key, (const int4*)c.ship_date,
+                   (const longlong2*)c.ext_price, (const int4*)c.discount, c.n_rows, p.ship_date_gt,
+                   (const uint32_t*)okbm, (const int32_t*)nullptr, od.key_max, (Q3Slot*)ht, (uint32_t*)hits,
+                   (const uint32_t*)nullptr, (uint32_t*)nullptr, (const uint32_t*)cap, (const uint32_t*)(cnt + 2));
+      return (int)GPUDB_OK;
+    }
     const unsigned g = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((c.n_rows + 256 * kProbeBatches - 1) / (256 * kProbeBatches), (uint64_t)sms * 8));
     GPUDB_LAUNCH(call, q3_probe_kernel, g, 256, 0, c.order_key, c.ship_date, c.ext_price, c.discount, c.n_rows,
