@@ -205,16 +205,64 @@ int Call::begin(size_t result_bytes) {
   }
   if (want_direct_ && !big_ && !dwork_ && ctx_->h_slots_dev)
     direct_ = ctx_->h_slots_dev + (size_t)slot_ * kSlotBytes;
-  else
-    GPUDB_CUDA(ctx_, cudaMemsetAsync(dslot_, 0, kSlotHeader + result_bytes, s_));
+  else if (const int rc = clear(dslot_, 0, kSlotHeader + result_bytes))
+    return rc;
   if (t_) {
-    // the timed region starts after the result slot is cleared: kernels (and copies) only
+    // the timed region: the call's fills, kernels and copies
     e0_ = event_get(ctx_);
     e1_ = event_get(ctx_);
     if (!e0_ || !e1_) return fail(ctx_, GPUDB_E_CUDA, "cudaEventCreate failed");
     GPUDB_CUDA(ctx_, cudaEventRecord(e0_, s_));
   }
   return GPUDB_OK;
+}
+
+// Every range in turn, all blocks on each: 16-byte stores (the ranges start on 16 bytes), the last
+// bytes one by one.
+static __global__ void __launch_bounds__(256) clear_ranges_kernel(ClearRanges r) {
+  const uint64_t t = (uint64_t)blockIdx.x * 256 + threadIdx.x, T = (uint64_t)gridDim.x * 256;
+  for (int i = 0; i < r.count; i++) {
+    uint4* q = reinterpret_cast<uint4*>(r.p[i]);
+    const uint4 v = make_uint4(r.v[i], r.v[i], r.v[i], r.v[i]);
+    for (uint64_t k = t; k < r.n[i] / 16; k += T) q[k] = v;
+    const uint64_t tail = r.n[i] / 16 * 16 + t;
+    if (tail < r.n[i]) r.p[i][tail] = (unsigned char)r.v[i];
+  }
+}
+
+int Call::clear(void* p, int value, size_t bytes) {
+  if (!bytes) return GPUDB_OK;
+  if (clears_.count == ClearRanges::kMax || (reinterpret_cast<uintptr_t>(p) & 15u)) {
+    const int rc = flush_clears();
+    if (rc) return rc;
+  }
+  if (reinterpret_cast<uintptr_t>(p) & 15u) {
+    GPUDB_CUDA(ctx_, cudaMemsetAsync(p, value, bytes, s_));
+    return GPUDB_OK;
+  }
+  const int i = clears_.count++;
+  clears_.p[i] = static_cast<unsigned char*>(p);
+  clears_.n[i] = bytes;
+  clears_.v[i] = (uint32_t)(value & 0xFF) * 0x01010101u;
+  return GPUDB_OK;
+}
+
+int Call::flush_clears() {
+  const int n = clears_.count;
+  if (!n) return GPUDB_OK;
+  clears_.count = 0;
+  if (n == 1) {
+    GPUDB_CUDA(ctx_, cudaMemsetAsync(clears_.p[0], (int)(clears_.v[0] & 0xFFu), clears_.n[0], s_));
+    return GPUDB_OK;
+  }
+  ClearRanges r = clears_;
+  r.count = n;
+  uint64_t most = 0;
+  for (int i = 0; i < n; i++) most = std::max(most, r.n[i]);
+  const unsigned grid = (unsigned)std::max<uint64_t>(
+      1, std::min<uint64_t>((most / 16 + 1023) / 1024, (uint64_t)ctx_->sm_count * 8));
+  clear_ranges_kernel<<<grid, 256, 0, s_>>>(r);   // (stands for memsets: not in the call's kernel count)
+  return check_launch("clear_ranges_kernel");
 }
 
 int Call::begin_direct(size_t result_bytes) {
@@ -230,6 +278,7 @@ int Call::check_launch(const char* name) {
 
 int Call::side_begin() {
   if (main_) return fail(ctx_, GPUDB_E_INVALID, "side stream already in use by this call");
+  if (const int rc = flush_clears()) return rc;   // before the fork
   GPUDB_CUDA(ctx_, cudaEventRecord(ctx_->fork_ev, s_));
   GPUDB_CUDA(ctx_, cudaStreamWaitEvent(ctx_->side_stream, ctx_->fork_ev, 0));
   main_ = s_;
@@ -255,6 +304,7 @@ int Call::side_join() {
 
 int Call::finish(size_t result_bytes, std::function<int(const uint8_t*)> convert) {
   side_end();   // (a stage that failed on the side stream may have left it selected)
+  if (const int rc = flush_clears()) return rc;   // a call without a launch
   if (t_) GPUDB_CUDA(ctx_, cudaEventRecord(e1_, s_));
   size_t bytes = kSlotHeader + result_bytes;
   // (a direct result is already in hslot_ when the kernel completes; its bytes crossed the

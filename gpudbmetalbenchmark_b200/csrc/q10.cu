@@ -226,10 +226,10 @@ extern "C" int gpudb_q10_returned(gpudb_ctx* ctx, const gpudb_customer* cu, cons
   if (!rc) rc = scratch(ctx, "q10.topk", (size_t)kTopkStateWords * 4, &tstate);
   if (!rc) rc = scratch(ctx, "q10.cand", (size_t)kTopkCandCap * sizeof(u128), &cand);
   if (rc) return rc;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(custbm, 0, (size_t)cwords * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(okbm, 0, (size_t)owords * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(rev, 0, ((size_t)cust_max + 1) * 8, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(tstate, 0, (size_t)kTopkStateWords * 4, s));
+  if ((rc = call.clear(custbm, 0, (size_t)cwords * 4))) return rc;
+  if ((rc = call.clear(okbm, 0, (size_t)owords * 4))) return rc;
+  if ((rc = call.clear(rev, 0, ((size_t)cust_max + 1) * 8))) return rc;
+  if ((rc = call.clear(tstate, 0, (size_t)kTopkStateWords * 4))) return rc;
   uint8_t* res = call.result<uint8_t>();
   if (cu->n_rows)
     GPUDB_LAUNCH(call, bitmap_build_kernel, grid_for(ctx, cu->n_rows, 1, 16), kThreads, 0, cu->cust_key, nullptr, -1,

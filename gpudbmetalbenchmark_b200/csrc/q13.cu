@@ -340,8 +340,8 @@ extern "C" int gpudb_q13_distribution(gpudb_ctx* ctx, const gpudb_customer* cu, 
   void *counts = nullptr, *hist = nullptr;
   if ((rc = scratch(ctx, "q13.counts", ((size_t)cust_max + 1) * 4, &counts))) return rc;
   if ((rc = scratch(ctx, "q13.hist", (size_t)kBins * 4, &hist))) return rc;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(counts, 0, ((size_t)cust_max + 1) * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(hist, 0, (size_t)kBins * 4, s));
+  if ((rc = call.clear(counts, 0, ((size_t)cust_max + 1) * 4))) return rc;
+  if ((rc = call.clear(hist, 0, (size_t)kBins * 4))) return rc;
   const int sms = ctx->sm_count;
   if (od->n_rows && cu->n_rows) {
     auto kern = long_words ? q13_count_kernel<true> : q13_count_kernel<false>;

@@ -734,10 +734,10 @@ int q3_radix(Call& call, const gpudb_customer& cu, const gpudb_orders& od, const
   if (!rc) rc = scratch(ctx, "q3.topk", (size_t)kTopkStateWords * 4, &tstate);
   if (rc) return rc;
   uint32_t* cnt = static_cast<uint32_t*>(count);   // [0] orders, [1] fact rows, [2] groups, [3] top-k capacity
-  GPUDB_CUDA(ctx, cudaMemsetAsync(bitmap, 0, (size_t)words * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(kset, 0, (size_t)kwords * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(count, 0, 16, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(tstate, 0, (size_t)kTopkStateWords * 4, s));
+  if ((rc = call.clear(bitmap, 0, (size_t)words * 4))) return rc;
+  if ((rc = call.clear(kset, 0, (size_t)kwords * 4))) return rc;
+  if ((rc = call.clear(count, 0, 16))) return rc;
+  if ((rc = call.clear(tstate, 0, (size_t)kTopkStateWords * 4))) return rc;
   const int sms = ctx->sm_count;
   auto grid = [&](uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 16)); };
   uint32_t* ks = static_cast<uint32_t*>(kset);
@@ -814,10 +814,10 @@ int q3_direct(Call& call, const gpudb_customer& cu, const gpudb_orders& od, cons
   if (!rc) rc = scratch(ctx, "q3.cand", (size_t)kTopkCandCap * sizeof(u128), &cand);
   if (rc) return rc;
   uint32_t* cnt = static_cast<uint32_t*>(count);   // [0] orders, [1] top-k capacity
-  GPUDB_CUDA(ctx, cudaMemsetAsync(bitmap, 0, (size_t)words * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(okbm, 0, okbm_bytes, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(count, 0, 16, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(tstate, 0, (size_t)kTopkStateWords * 4, s));
+  if ((rc = call.clear(bitmap, 0, (size_t)words * 4))) return rc;
+  if ((rc = call.clear(okbm, 0, okbm_bytes))) return rc;
+  if ((rc = call.clear(count, 0, 16))) return rc;
+  if ((rc = call.clear(tstate, 0, (size_t)kTopkStateWords * 4))) return rc;
   const int sms = ctx->sm_count;
   if (cu.n_rows) {
     const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((cu.n_rows + 255) / 256, (uint64_t)sms * 16));
@@ -894,10 +894,10 @@ int q3_global(Call& call, const gpudb_customer& cu, const gpudb_orders& od, cons
   if (rc) return rc;
   uint32_t* cnt = static_cast<uint32_t*>(count);
   uint32_t* cap = cnt + 1;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(bitmap, 0, (size_t)words * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(count, 0, 16, s));   // [0] count, [1] capacity, [2] okbm off, [3] ticket
-  if (use_okbm) GPUDB_CUDA(ctx, cudaMemsetAsync(okbm, 0, okbm_bytes, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(tstate, 0, (size_t)kTopkStateWords * 4, s));
+  if ((rc = call.clear(bitmap, 0, (size_t)words * 4))) return rc;
+  if ((rc = call.clear(count, 0, 16))) return rc;   // [0] count, [1] capacity, [2] okbm off, [3] ticket
+  if (use_okbm) if ((rc = call.clear(okbm, 0, okbm_bytes))) return rc;
+  if ((rc = call.clear(tstate, 0, (size_t)kTopkStateWords * 4))) return rc;
   const int sms = ctx->sm_count;
   auto grid = [&](uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 16)); };
   if (cu.n_rows)

@@ -320,10 +320,10 @@ int q3_batch_run(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32_t
   m.hits = static_cast<uint32_t*>(hits);
   m.cand = static_cast<u128*>(cand);
   m.tstate = static_cast<uint32_t*>(tstate);
-  GPUDB_CUDA(ctx, cudaMemsetAsync(bm, 0, (size_t)m.D * m.words * 4, s));
-  if (use_okbm) GPUDB_CUDA(ctx, cudaMemsetAsync(okbm, 0, (size_t)K * m.okwords * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(cnt, 0, (4 * kB + 1) * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(tstate, 0, (size_t)K * kTopkStateWords * 4, s));
+  if ((rc = call.clear(bm, 0, (size_t)m.D * m.words * 4))) return rc;
+  if (use_okbm) if ((rc = call.clear(okbm, 0, (size_t)K * m.okwords * 4))) return rc;
+  if ((rc = call.clear(cnt, 0, (4 * kB + 1) * 4))) return rc;
+  if ((rc = call.clear(tstate, 0, (size_t)K * kTopkStateWords * 4))) return rc;
   const int sms = ctx->sm_count;
   auto grid = [&](uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 16)); };
   GPUDB_LAUNCH(call, q3m_bitmap_kernel, dim3(grid(cu.n_rows), m.D), 256, 0, cu.cust_key, cu.segment, cu.n_rows, cu.key_max, m);

@@ -196,7 +196,7 @@ extern "C" int gpudb_q4_priority(gpudb_ctx* ctx, const gpudb_orders* od, const g
   const uint32_t words = (uint32_t)(key_max >> 5) + 1;
   void* bits = nullptr;
   if ((rc = scratch(ctx, "q4.late", (size_t)words * 4, &bits))) return rc;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(bits, 0, (size_t)words * 4, s));
+  if ((rc = call.clear(bits, 0, (size_t)words * 4))) return rc;
   if (od->n_rows) {
     rc = stream_lineitem(call, li, mask, 0, [&](const gpudb_lineitem& c) {
       if (c.n_rows)
@@ -231,7 +231,7 @@ extern "C" int gpudb_q12_shipmode(gpudb_ctx* ctx, const gpudb_orders* od, const 
   const uint32_t words = (uint32_t)(key_max >> 5) + 1;
   void* bits = nullptr;
   if ((rc = scratch(ctx, "q12.high", (size_t)words * 4, &bits))) return rc;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(bits, 0, (size_t)words * 4, s));
+  if ((rc = call.clear(bits, 0, (size_t)words * 4))) return rc;
   if (od->n_rows)
     GPUDB_LAUNCH(call, q12_prio_kernel, scan_grid(ctx, od->n_rows), kThreads, 0, od->order_key, od->priority,
                  od->n_rows, p->high_max, key_max, (uint32_t*)bits, call.status());

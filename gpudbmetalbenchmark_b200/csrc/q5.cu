@@ -138,9 +138,9 @@ extern "C" int gpudb_q5_local_supplier(gpudb_ctx* ctx, const gpudb_customer* cu,
   if (!rc) rc = scratch(ctx, "q5.okbm", (size_t)owords * 4, &okbm);
   if (!rc) rc = scratch(ctx, "q5.omap", (size_t)order_max + 1, &omap);
   if (rc) return rc;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(cmap, kNone, (size_t)cust_max + 1, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(smap, kNone, (size_t)supp_max + 1, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(okbm, 0, (size_t)owords * 4, s));
+  if ((rc = call.clear(cmap, kNone, (size_t)cust_max + 1))) return rc;
+  if ((rc = call.clear(smap, kNone, (size_t)supp_max + 1))) return rc;
+  if ((rc = call.clear(okbm, 0, (size_t)owords * 4))) return rc;
   if (cu->n_rows)
     GPUDB_LAUNCH(call, nation_map_kernel, grid_for(ctx, cu->n_rows, 1, 8), kThreads, 0, cu->cust_key, cu->nation,
                  cu->n_rows, cust_max, p->nation_mask, (uint8_t*)cmap, call.status());

@@ -299,9 +299,9 @@ extern "C" int gpudb_q7_volume_shipping(gpudb_ctx* ctx, const gpudb_customer* cu
   if (!rc) rc = scratch(ctx, "q7.okbm", (size_t)owords * 4, &okbm);
   if (!rc) rc = scratch(ctx, "q7.omap", (size_t)order_max + 1, &omap);
   if (rc) return rc;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(cmap, kNone, (size_t)cust_max + 1, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(smap, kNone, (size_t)supp_max + 1, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(okbm, 0, (size_t)owords * 4, s));
+  if ((rc = call.clear(cmap, kNone, (size_t)cust_max + 1))) return rc;
+  if ((rc = call.clear(smap, kNone, (size_t)supp_max + 1))) return rc;
+  if ((rc = call.clear(okbm, 0, (size_t)owords * 4))) return rc;
   const uint32_t pair_mask = (1u << p->nation_a) | (1u << p->nation_b);
   if (cu->n_rows)
     GPUDB_LAUNCH(call, nation_map_kernel, grid_for(ctx, cu->n_rows, 1, 8), kThreads, 0, cu->cust_key, cu->nation,
@@ -366,10 +366,10 @@ extern "C" int gpudb_q8_market_share(gpudb_ctx* ctx, const gpudb_customer* cu, c
   if (!rc) rc = scratch(ctx, "q8.omap", (size_t)order_max + 1, &omap);
   if (!rc) rc = scratch(ctx, "q8.pbits", (size_t)pwords * 4, &pbits);
   if (rc) return rc;
-  GPUDB_CUDA(ctx, cudaMemsetAsync(cmap, kNone, (size_t)cust_max + 1, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(smap, kNone, (size_t)supp_max + 1, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(okbm, 0, (size_t)owords * 4, s));
-  GPUDB_CUDA(ctx, cudaMemsetAsync(pbits, 0, (size_t)pwords * 4, s));
+  if ((rc = call.clear(cmap, kNone, (size_t)cust_max + 1))) return rc;
+  if ((rc = call.clear(smap, kNone, (size_t)supp_max + 1))) return rc;
+  if ((rc = call.clear(okbm, 0, (size_t)owords * 4))) return rc;
+  if ((rc = call.clear(pbits, 0, (size_t)pwords * 4))) return rc;
   if (pa->n_rows)
     GPUDB_LAUNCH(call, bitmap_build_kernel, grid_for(ctx, pa->n_rows, 1, 16), kThreads, 0, pa->part_key, pa->type,
                  p->part_type, pa->n_rows, part_max, (uint32_t*)pbits, call.status());
@@ -391,7 +391,7 @@ extern "C" int gpudb_q8_market_share(gpudb_ctx* ctx, const gpudb_customer* cu, c
     void* hfilt = nullptr;
     if (!exact) {
       if ((rc = scratch(ctx, "q8.partfilter", (size_t)kSmemFilterWords * 4, &hfilt))) return rc;
-      GPUDB_CUDA(ctx, cudaMemsetAsync(hfilt, 0, (size_t)kSmemFilterWords * 4, s));
+      if ((rc = call.clear(hfilt, 0, (size_t)kSmemFilterWords * 4))) return rc;
       GPUDB_LAUNCH(call, hashed_filter_kernel, grid_for(ctx, pwords, 1, 8), kThreads, 0, (const uint32_t*)pbits, pwords,
                    (uint32_t*)hfilt);
     }

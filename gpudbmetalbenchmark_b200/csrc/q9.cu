@@ -442,6 +442,7 @@ extern "C" int gpudb_q9_star(gpudb_ctx* ctx, const gpudb_part* pa, const gpudb_s
   Call call(ctx, ex, t);
   const size_t bytes = 16 + (size_t)gcap * 16;
   if ((rc = call.begin(bytes))) return rc;
+  if ((rc = call.flush_clears())) return rc;   // the slot's, before any capture
   cudaStream_t s = call.stream();
   const int32_t part_max = pa->n_rows ? pa->key_max : 0, supp_max = su->n_rows ? su->key_max : 0;
   const int32_t order_max = od->n_rows ? od->key_max : 0;
