@@ -137,6 +137,29 @@ __device__ __forceinline__ uint32_t smem_filter_mask(const uint32_t* sfilt, bool
   return pass & hit;
 }
 
+// Sets the bits key[j] of `bitmap` for the rows j of `on` (four rows a lane, keys already
+// range-checked). A lane merges its rows of one word (four rows in a row are of one order or of
+// neighbours), and the lanes of a word are merged (__match_any_sync, a masked OR-reduce) into
+// one atomicOr; a lane's rows of another word go by themselves. For bitmaps most rows set; where
+// few do (the reports' windows and nations), one row a lane at a time is as fast.
+// Every lane of the warp calls it.
+__device__ __forceinline__ void warp_bitmap_or4(uint32_t on, const int32_t (&key)[4], uint32_t* bitmap) {
+  uint32_t word = ~0u, bits = 0;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const uint32_t w = (uint32_t)key[j] >> 5, bit = 1u << ((uint32_t)key[j] & 31u);
+    if (!((on >> j) & 1u)) continue;
+    if (word == ~0u) word = w;
+    if (word == w) bits |= bit;
+    else atomicOr(bitmap + w, bit);
+  }
+  const uint32_t onmask = __ballot_sync(FULL_MASK, bits != 0);
+  if (!bits) return;
+  const uint32_t peers = __match_any_sync(onmask, word);
+  const uint32_t all = __reduce_or_sync(peers, bits);
+  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicOr(bitmap + word, all);
+}
+
 // Sets bit `key` of `bitmap` for the lanes with `on` (keys already range-checked): one
 // atomicOr per distinct word of the warp (lanes of a word found with __match_any_sync, their
 // bits merged with a masked OR-reduce). Every lane of the warp calls it.
