@@ -171,7 +171,7 @@ struct Q9Maps {
 constexpr int kQ9Threads = 256;
 
 constexpr int kLiThreads = 1024;
-constexpr int kLiQuads = 4;                  // 128-row groups per warp per block step
+constexpr int kLiQuads = 2;                  // 128-row groups per warp per block step
 constexpr int kLiRows = 4 * kLiQuads;        // fact rows per thread per block step of li_filter_kernel
 constexpr uint64_t kQ9Piece = 64ull << 20;   // fact rows per filter + resolve pair (bounds the pair buffer)
 
@@ -182,7 +182,7 @@ enum : int {
 };
 
 // Fact rows whose part passes the filter -> bit (r & 31) of passbits[r >> 5] (rows of the
-// piece). A block step covers kLiThreads * 16 rows in 128-row groups, four per warp; lane L
+// piece). A block step covers kLiThreads * 8 rows in 128-row groups, two per warp; lane L
 // tests rows 32k + L of a group (k = 0..3), loaded by four coalesced 4-byte loads (128 bytes
 // a warp each, any alignment), so the vote (__ballot_sync) of the lanes' row-32k tests is the
 // bitmask word k itself: one instruction a word, no shuffles, and lane 0 stores the group's
@@ -191,8 +191,12 @@ enum : int {
 // kPartBloom a blocked Bloom filter in shared memory, whose word index is in range for any
 // key and whose hits (false positives, and keys outside the part range) the resolve
 // confirms against the exact bitmap.
+// 32 registers a thread (two groups in flight): half of an SM's registers stay free for the side
+// stream's kernels beside the filter's 200 KB of shared memory. Whole call at 60M fact rows: 535
+// us with four groups and 51 registers, 529 us so; with the side kernels asking for the same
+// shared-memory split 543 us (they lose their L1).
 template <int MODE>
-__global__ void __launch_bounds__(kLiThreads) li_filter_kernel(const int32_t* __restrict__ part, uint64_t n,
+__global__ void __launch_bounds__(kLiThreads, 2) li_filter_kernel(const int32_t* __restrict__ part, uint64_t n,
                                                                int32_t part_max, const uint32_t* __restrict__ filt,
                                                                uint32_t filt_words, uint32_t* __restrict__ passbits) {
   extern __shared__ uint32_t sfilt[];
@@ -442,7 +446,6 @@ extern "C" int gpudb_q9_star(gpudb_ctx* ctx, const gpudb_part* pa, const gpudb_s
   Call call(ctx, ex, t);
   const size_t bytes = 16 + (size_t)gcap * 16;
   if ((rc = call.begin(bytes))) return rc;
-  if ((rc = call.flush_clears())) return rc;   // the slot's, before any capture
   cudaStream_t s = call.stream();
   const int32_t part_max = pa->n_rows ? pa->key_max : 0, supp_max = su->n_rows ? su->key_max : 0;
   const int32_t order_max = od->n_rows ? od->key_max : 0;
