@@ -173,7 +173,7 @@ Call::~Call() {
   }
 }
 
-int Call::begin(size_t result_bytes) {
+int Call::begin(size_t result_bytes, bool defer) {
   // a non-sticky error left by earlier, unrelated runtime calls is not this call's (a
   // sticky one still shows at this call's first launch)
   (void)cudaGetLastError();
@@ -207,6 +207,8 @@ int Call::begin(size_t result_bytes) {
     direct_ = ctx_->h_slots_dev + (size_t)slot_ * kSlotBytes;
   else if (const int rc = clear(dslot_, 0, kSlotHeader + result_bytes))
     return rc;
+  if (!defer)
+    if (const int rc = flush_clears()) return rc;
   if (t_) {
     // the timed region: the call's fills, kernels and copies
     e0_ = event_get(ctx_);

@@ -148,10 +148,13 @@ class Call {
  public:
   Call(gpudb_ctx* ctx, const gpudb_exec* ex, gpudb_timing* t);
   ~Call();
-  int begin(size_t result_bytes);          // acquires a slot; header + payload are zero before the first launch
+  // Acquires a slot; header + payload are zero before the first launch: cleared at once, or
+  // (`defer`) with the fills the pipeline asks for next (clear).
+  int begin(size_t result_bytes, bool defer = false);
   // Fills `bytes` at `p` with the byte `value` before the call's next kernel launch. The fills a
   // pipeline asks for at its start (its slot's among them) go as one kernel: a memset each took
-  // about 1.5 us, five of them in a Q3 call.
+  // about 1.5 us, five of them in a Q3 call. (A pipeline with no fill of its own clears its slot
+  // at once, while the host prepares the launch: deferred, it cost such a call 0.9 us.)
   int clear(void* p, int value, size_t bytes);
   int flush_clears();
   // Direct result: for a pipeline whose result comes from ONE kernel's last block. The slot

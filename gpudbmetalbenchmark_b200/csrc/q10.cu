@@ -214,7 +214,7 @@ extern "C" int gpudb_q10_returned(gpudb_ctx* ctx, const gpudb_customer* cu, cons
   if (rc) return rc;
   Call call(ctx, ex, t);
   const size_t bytes = 16 + (size_t)GPUDB_Q3_MAX_K * sizeof(u128);
-  if ((rc = call.begin(bytes))) return rc;
+  if ((rc = call.begin(bytes, true))) return rc;
   cudaStream_t s = call.stream();
   const int32_t cust_max = cu->n_rows ? cu->key_max : 0, order_max = od->n_rows ? od->key_max : 0;
   const uint32_t cwords = (uint32_t)(cust_max >> 5) + 1, owords = (uint32_t)(order_max >> 5) + 1;

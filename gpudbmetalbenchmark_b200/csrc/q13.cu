@@ -333,7 +333,7 @@ extern "C" int gpudb_q13_distribution(gpudb_ctx* ctx, const gpudb_customer* cu, 
   const bool long_words = pat.len[0] >= kLongWord && pat.len[1] >= kLongWord;
   Call call(ctx, ex, t);
   const size_t bytes = 16 + (size_t)kBins * sizeof(gpudb_q13_row);
-  int rc = call.begin(bytes);
+  int rc = call.begin(bytes, true);
   if (rc) return rc;
   cudaStream_t s = call.stream();
   const int32_t cust_max = cu->n_rows ? cu->key_max : 0;

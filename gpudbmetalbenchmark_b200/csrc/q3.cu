@@ -977,7 +977,7 @@ extern "C" int gpudb_q3_join_topk(gpudb_ctx* ctx, const gpudb_customer* cu, cons
     return fail(ctx, GPUDB_E_INVALID, "q3: the direct mode needs orders.key_max");
   Call call(ctx, ex, t);
   const size_t bytes = 16 + (size_t)GPUDB_Q3_MAX_K * sizeof(u128);
-  if ((rc = call.begin(bytes))) return rc;
+  if ((rc = call.begin(bytes, true))) return rc;
   uint8_t* res = call.result<uint8_t>();
   rc = mode == GPUDB_JOIN_GLOBAL ? q3_global(call, c, o, li, pp, res)
      : mode == GPUDB_JOIN_DIRECT ? q3_direct(call, c, o, li, pp, res)

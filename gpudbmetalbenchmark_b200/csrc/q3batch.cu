@@ -310,7 +310,7 @@ int q3_batch_run(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32_t
   // result slot: K status words, D segment status words, K payloads
   const size_t st_bytes = 64, bytes = st_bytes + (size_t)K * kReqBytes;
   Call call(ctx, ex, nullptr);
-  int rc = call.begin(bytes);
+  int rc = call.begin(bytes, true);
   if (rc) return rc;
   cudaStream_t s = call.stream();
   uint8_t* res = call.result<uint8_t>();

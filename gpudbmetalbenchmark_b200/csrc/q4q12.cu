@@ -182,7 +182,7 @@ extern "C" int gpudb_q4_priority(gpudb_ctx* ctx, const gpudb_orders* od, const g
   if (!rc) rc = lineitem_check(ctx, li, mask);
   if (rc) return rc;
   Call call(ctx, ex, t);
-  if ((rc = call.begin(40))) return rc;
+  if ((rc = call.begin(40, true))) return rc;
   cudaStream_t s = call.stream();
   const int32_t key_max = od->n_rows ? od->key_max : 0;
   const uint32_t words = (uint32_t)(key_max >> 5) + 1;
@@ -217,7 +217,7 @@ extern "C" int gpudb_q12_shipmode(gpudb_ctx* ctx, const gpudb_orders* od, const 
   if (!rc) rc = lineitem_check(ctx, li, mask);
   if (rc) return rc;
   Call call(ctx, ex, t);
-  if ((rc = call.begin(32))) return rc;
+  if ((rc = call.begin(32, true))) return rc;
   cudaStream_t s = call.stream();
   const int32_t key_max = od->n_rows ? od->key_max : 0;
   const uint32_t words = (uint32_t)(key_max >> 5) + 1;

@@ -127,7 +127,7 @@ extern "C" int gpudb_q5_local_supplier(gpudb_ctx* ctx, const gpudb_customer* cu,
   int rc = lineitem_check(ctx, li, mask);
   if (rc) return rc;
   Call call(ctx, ex, t);
-  if ((rc = call.begin(GPUDB_NATIONS * 8))) return rc;
+  if ((rc = call.begin(GPUDB_NATIONS * 8, true))) return rc;
   cudaStream_t s = call.stream();
   const int32_t cust_max = cu->n_rows ? cu->key_max : 0, supp_max = su->n_rows ? su->key_max : 0;
   const int32_t order_max = od->n_rows ? od->key_max : 0;

@@ -288,7 +288,7 @@ extern "C" int gpudb_q7_volume_shipping(gpudb_ctx* ctx, const gpudb_customer* cu
   if (rc) return rc;
   Call call(ctx, ex, t);
   const size_t bytes = 2 * kYears * 8;
-  if ((rc = call.begin(bytes))) return rc;
+  if ((rc = call.begin(bytes, true))) return rc;
   cudaStream_t s = call.stream();
   const int32_t cust_max = cu->n_rows ? cu->key_max : 0, supp_max = su->n_rows ? su->key_max : 0;
   const int32_t order_max = od->n_rows ? od->key_max : 0;
@@ -354,7 +354,7 @@ extern "C" int gpudb_q8_market_share(gpudb_ctx* ctx, const gpudb_customer* cu, c
   if (rc) return rc;
   Call call(ctx, ex, t);
   const size_t bytes = 2 * kYears * 8;
-  if ((rc = call.begin(bytes))) return rc;
+  if ((rc = call.begin(bytes, true))) return rc;
   cudaStream_t s = call.stream();
   const int32_t cust_max = cu->n_rows ? cu->key_max : 0, supp_max = su->n_rows ? su->key_max : 0;
   const int32_t order_max = od->n_rows ? od->key_max : 0, part_max = pa->n_rows ? pa->key_max : 0;

@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(kQ1SmemThreads, MINB) q1_vec_smem_kernel(const
 #pragma unroll
   for (int r = 0; r < NQ6; r++) { rrev[r] = 0; rcnt[r] = 0; }
   auto row = [&](int32_t s, int32_t qt, int64_t e, int32_t d, int32_t tx, uint32_t f, uint32_t st) {
-    const uint64_t ed = (uint64_t)(e * (int64_t)d);
+    const uint64_t ed = NQ6 > 0 ? (uint64_t)(e * (int64_t)d) : (uint64_t)e * (uint32_t)d;
 #pragma unroll
     for (int r = 0; r < NQ6; r++) {
       const bool m = q6_pass(s, d, qt, riders.p[r]);
