@@ -832,10 +832,12 @@ int launch_q6(Call& call, const gpudb_lineitem& c, const gpudb_q6_params& p, voi
   const Q6P pp{p.ship_lo, p.ship_hi, p.disc_lo, p.disc_hi, p.qty_lt};
   const bool vec = aligned(c.ship_date, 16) && aligned(c.discount, 16) && aligned(c.quantity, 16) && aligned(c.ext_price, 8);
   // 1 one row per thread; 2/3/4: 128-bit loads, 1/2/4 quads per thread per step. Auto (0): one
-  // quad per step, but one row per thread for 2^21..2^22 rows, where the columns stay in L2
-  // across calls and a quad grid ends in a short wave (3M rows: 22.7 us a call against 23.8;
-  // 1M: 19.0 against 17.8, 6M: 37.4 against 31.1, 12M: 56 against 44; two tables in turn)
-  int variant = ctx->q6_variant ? ctx->q6_variant : (c.n_rows >= (1u << 21) && c.n_rows < (1u << 22) ? 1 : 2);
+  // quad per step, but one row per thread from 2^21 rows while the columns (20 B a row) fit the
+  // 126 MB L2: over one table that stays there the row form is ahead (6M rows 20.4 us against
+  // 23.2, 3M 22.7 against 23.8 a call), below and above it is not (two tables in turn: 1M rows
+  // 19.0 us against 17.8, 12M 56 against 44)
+  int variant = ctx->q6_variant ? ctx->q6_variant
+                                : (c.n_rows >= (1u << 21) && c.n_rows * 20 <= (126ull << 20) ? 1 : 2);
   if (!vec) variant = 1;
   const int unroll = variant == 2 ? 1 : variant == 4 ? 4 : 2;
   const void* kfn = variant == 1 ? (const void*)q6_row_kernel
@@ -967,6 +969,19 @@ int launch_q1(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, voi
   return GPUDB_OK;
 }
 
+static constexpr Q1SmemKernel kRiding[2][kMaxRiders + 1] = {
+    {q1_vec_smem_kernel<2, 0>, q1_vec_smem_kernel<2, 1>, q1_vec_smem_kernel<2, 2>, q1_vec_smem_kernel<2, 3>,
+     q1_vec_smem_kernel<2, 4>},
+    {q1_vec_smem_kernel<2, 0, 2, 2>, q1_vec_smem_kernel<2, 1, 2, 2>, q1_vec_smem_kernel<2, 2, 2, 2>,
+     q1_vec_smem_kernel<2, 3, 2, 2>, q1_vec_smem_kernel<2, 4, 2, 2>}};
+
+int load_scan_kernels(gpudb_ctx* ctx) {
+  for (int j = 0; j < 2; j++)
+    for (Q1SmemKernel k : kRiding[j]) GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)k, kQ1AccBytes * (j + 1)));
+  for (const void* k : {(const void*)q6_row_kernel, (const void*)q6_vec_kernel<1>}) GPUDB_CUDA(ctx, kernel_smem(ctx, k, 16));
+  return GPUDB_OK;
+}
+
 bool q1_shared_ok(const gpudb_ctx* ctx, const gpudb_lineitem& c) {
   return aligned(c.ship_date, 16) && aligned(c.quantity, 16) && aligned(c.ext_price, 16) && aligned(c.discount, 16) &&
          aligned(c.tax, 16) && aligned(c.flag, 4) && aligned(c.status, 4) && c.n_rows > 0 && ctx->scan_variant == 0;
@@ -995,11 +1010,6 @@ int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1
       rq.status[j] = q1status[r];
     }
   }
-  static constexpr Q1SmemKernel kRiding[2][kMaxRiders + 1] = {
-      {q1_vec_smem_kernel<2, 0>, q1_vec_smem_kernel<2, 1>, q1_vec_smem_kernel<2, 2>, q1_vec_smem_kernel<2, 3>,
-       q1_vec_smem_kernel<2, 4>},
-      {q1_vec_smem_kernel<2, 0, 2, 2>, q1_vec_smem_kernel<2, 1, 2, 2>, q1_vec_smem_kernel<2, 2, 2, 2>,
-       q1_vec_smem_kernel<2, 3, 2, 2>, q1_vec_smem_kernel<2, 4, 2, 2>}};
   return launch_q1_smem(call, c, rq, n1, kRiding[n1 - 1][n6], rd);
 }
 

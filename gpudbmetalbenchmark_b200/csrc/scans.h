@@ -24,6 +24,10 @@ int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1
 // Whether launch_q1_riders would share one read of these columns between requests.
 bool q1_shared_ok(const gpudb_ctx* ctx, const gpudb_lineitem& c);
 
+// Loads the scan kernels a batch may use. The runtime loads a kernel at its first use, which would
+// hold up a served stream when a batch first has a new mix of requests.
+int load_scan_kernels(gpudb_ctx* ctx);
+
 // Host result from the kQ1ResultBytes device words of one Q1 scan.
 void q1_result_from(const uint8_t* words, gpudb_q1_result* out);
 
