@@ -268,15 +268,18 @@ __device__ __forceinline__ void red_add_limbs(unsigned long long* w, u128 v) {
 // next launch (it is zero when first allocated). No per-block partials are read back.
 // NQ1 = 2: the sums come in two buckets of 24 columns (rows up to the first request's cutoff, rows
 // between the cutoffs), `bad` in bit j for bucket j; the second request's totals are both.
+// Sized by NQ1: one request through the two-request form costs a call 0.7 us (3M rows 36.8 us
+// against 36.0), at every size.
+template <int NQ1>
 struct Q1Requests {
-  int32_t cut[2];          // ship_date cutoffs, ascending
-  u128* out[2];
-  uint32_t* status[2];
+  int32_t cut[NQ1];        // ship_date cutoffs, ascending
+  u128* out[NQ1];
+  uint32_t* status[NQ1];
 };
 
 template <int T, int NQ1>
 __device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, unsigned long long* gacc, unsigned* ticket,
-                                             const Q1Requests& rq, uint32_t* hstatus) {
+                                             const Q1Requests<NQ1>& rq, uint32_t* hstatus) {
   constexpr int W = T / 32;
   static_assert(24 % W == 0, "whole columns per warp");
   __shared__ u128 tot[NQ1 * 6 * kQ1Raw];
@@ -286,7 +289,7 @@ __device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, 
   for (int j = 0; j < NQ1; j++)
     if (__syncthreads_or(bad & ((2u << j) - 1u)) && threadIdx.x == 0) set_status(rq.status[j], ST_DOMAIN);
   for (int c = warp; c < NQ1 * 24; c += W) {
-    const int metric = c % 24 / 6, g = c / 24 * 6 + c % 6;   // g: bucket and group
+    const int metric = NQ1 > 1 ? c % 24 / 6 : c / 6, g = NQ1 > 1 ? c / 24 * 6 + c % 6 : c % 6;   // g: bucket and group
     u128 s0 = 0, s1 = 0, s2 = 0;
 #pragma unroll 4
     for (int i = lane; i < T; i += 32) {
@@ -332,11 +335,14 @@ __device__ __forceinline__ void q1_smem_fold(const uint64_t* acc, uint32_t bad, 
   __syncthreads();
   if (threadIdx.x < NQ1 * 6) {
     const int j = NQ1 > 1 ? threadIdx.x / 6 : 0, g = threadIdx.x - 6 * j;
-    u128 r[kQ1Raw];
+    u128* const r = tot + threadIdx.x * kQ1Raw;
+    if (NQ1 > 1) {   // both buckets are the second request's
+      const u128* a = tot + g * kQ1Raw;
 #pragma unroll
-    for (int m = 0; m < kQ1Raw; m++) {
-      r[m] = tot[g * kQ1Raw + m];
-      if (NQ1 > 1 && j) r[m] += tot[(6 + g) * kQ1Raw + m];
+      for (int m = 0; m < kQ1Raw; m++) {
+        const u128 lo = a[m];
+        if (j) r[m] += lo;
+      }
     }
     const u128 disc_price = (u128)100 * r[2] - r[3];
     const u128 charge = (u128)100 * disc_price + r[4];
@@ -716,7 +722,7 @@ template <int MINB, int NQ6, int QPI = 2, int NQ1 = 1>
 __global__ void __launch_bounds__(kQ1SmemThreads, MINB) q1_vec_smem_kernel(const int4* __restrict__ ship4, const int4* __restrict__ qty4,
                                                                      const longlong2* __restrict__ ext2, const int4* __restrict__ disc4,
                                                                      const int4* __restrict__ tax4, const uint32_t* __restrict__ flag4,
-                                                                     const uint32_t* __restrict__ stat4, uint64_t n, Q1Requests rq,
+                                                                     const uint32_t* __restrict__ stat4, uint64_t n, Q1Requests<NQ1> rq,
                                                                      unsigned long long* gacc, unsigned* ticket,
                                                                      uint32_t* hstatus, Q6Riders riders) {
   constexpr int T = kQ1SmemThreads;
@@ -867,12 +873,14 @@ int launch_q6(Call& call, const gpudb_lineitem& c, const gpudb_q6_params& p, voi
 // With `hstatus` (a direct result: `out` and `hstatus` in the call's mapped host slot) the
 // launch's status word is the one in the scratch header beside the ticket, which the last
 // block copies to the host slot and leaves at zero.
+template <int NQ1>
 using Q1SmemKernel = void (*)(const int4*, const int4*, const longlong2*, const int4*, const int4*, const uint32_t*,
-                              const uint32_t*, uint64_t, Q1Requests, unsigned long long*, unsigned*, uint32_t*, Q6Riders);
-static int launch_q1_smem(Call& call, const gpudb_lineitem& c, Q1Requests rq, int nq1, Q1SmemKernel kern,
+                              const uint32_t*, uint64_t, Q1Requests<NQ1>, unsigned long long*, unsigned*, uint32_t*, Q6Riders);
+template <int NQ1>
+static int launch_q1_smem(Call& call, const gpudb_lineitem& c, Q1Requests<NQ1> rq, Q1SmemKernel<NQ1> kern,
                           const Q6Riders& riders, uint32_t* hstatus = nullptr) {
   gpudb_ctx* ctx = call.ctx();
-  const size_t smem = kQ1AccBytes * nq1;
+  const size_t smem = kQ1AccBytes * NQ1;
   GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)kern, smem));
   const int per_sm = kernel_occupancy(ctx, (const void*)kern, kQ1SmemThreads, smem);
   const uint64_t min_blocks = (c.n_rows + (uint64_t)kQ1SmemThreads * kQ1RowsPerThread - 1) /
@@ -906,11 +914,11 @@ static int q1_variant(const gpudb_ctx* ctx, const gpudb_lineitem& c) {
   return variant;
 }
 
-static Q1Requests q1_one(const gpudb_q1_params& p, void* out, uint32_t* status) {
-  return Q1Requests{{p.ship_le, 0}, {static_cast<u128*>(out), nullptr}, {status, nullptr}};
+static Q1Requests<1> q1_one(const gpudb_q1_params& p, void* out, uint32_t* status) {
+  return Q1Requests<1>{{p.ship_le}, {static_cast<u128*>(out)}, {status}};
 }
 
-static Q1SmemKernel q1_smem_kernel(int variant) {
+static Q1SmemKernel<1> q1_smem_kernel(int variant) {
   return variant == 8  ? q1_vec_smem_kernel<3, 0, 2>
        : variant == 9  ? q1_vec_smem_kernel<2, 0, 4>
        : variant == 10 ? q1_vec_smem_kernel<4, 0, 1>
@@ -924,7 +932,7 @@ int launch_q1(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, voi
   // 0 auto, 1 TMA 2048-row tiles x 4 stages, 2 vector loads, 3 one row per thread,
   // 4 TMA 4096-row tiles x 2 stages, 5/6 TMA rings, 7-10 shared-memory sums
   const int variant = q1_variant(ctx, c);
-  if (variant >= 7 && variant <= 10) return launch_q1_smem(call, c, q1_one(p, out, status), 1, q1_smem_kernel(variant), Q6Riders{});
+  if (variant >= 7 && variant <= 10) return launch_q1_smem(call, c, q1_one(p, out, status), q1_smem_kernel(variant), Q6Riders{});
   if (variant == 1 || variant >= 4) {
     const uint32_t R = (variant == 1 || variant == 5) ? 2048u : variant == 6 ? 1024u : 4096u;
     const int threads = variant == 6 ? 256 : kQ1TmaThreads;
@@ -969,15 +977,16 @@ int launch_q1(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, voi
   return GPUDB_OK;
 }
 
-static constexpr Q1SmemKernel kRiding[2][kMaxRiders + 1] = {
-    {q1_vec_smem_kernel<2, 0>, q1_vec_smem_kernel<2, 1>, q1_vec_smem_kernel<2, 2>, q1_vec_smem_kernel<2, 3>,
-     q1_vec_smem_kernel<2, 4>},
-    {q1_vec_smem_kernel<2, 0, 2, 2>, q1_vec_smem_kernel<2, 1, 2, 2>, q1_vec_smem_kernel<2, 2, 2, 2>,
-     q1_vec_smem_kernel<2, 3, 2, 2>, q1_vec_smem_kernel<2, 4, 2, 2>}};
+static constexpr Q1SmemKernel<1> kRiding[kMaxRiders + 1] = {q1_vec_smem_kernel<2, 0>, q1_vec_smem_kernel<2, 1>,
+                                                            q1_vec_smem_kernel<2, 2>, q1_vec_smem_kernel<2, 3>,
+                                                            q1_vec_smem_kernel<2, 4>};
+static constexpr Q1SmemKernel<2> kRiding2[kMaxRiders + 1] = {q1_vec_smem_kernel<2, 0, 2, 2>, q1_vec_smem_kernel<2, 1, 2, 2>,
+                                                             q1_vec_smem_kernel<2, 2, 2, 2>, q1_vec_smem_kernel<2, 3, 2, 2>,
+                                                             q1_vec_smem_kernel<2, 4, 2, 2>};
 
 int load_scan_kernels(gpudb_ctx* ctx) {
-  for (int j = 0; j < 2; j++)
-    for (Q1SmemKernel k : kRiding[j]) GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)k, kQ1AccBytes * (j + 1)));
+  for (Q1SmemKernel<1> k : kRiding) GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)k, kQ1AccBytes));
+  for (Q1SmemKernel<2> k : kRiding2) GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)k, kQ1AccBytes * 2));
   for (const void* k : {(const void*)q6_row_kernel, (const void*)q6_vec_kernel<1>}) GPUDB_CUDA(ctx, kernel_smem(ctx, k, 16));
   return GPUDB_OK;
 }
@@ -1000,17 +1009,16 @@ int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1
     rd.p[r] = Q6P{q6[r].ship_lo, q6[r].ship_hi, q6[r].disc_lo, q6[r].disc_hi, q6[r].qty_lt};
     rd.out[r] = static_cast<unsigned long long*>(q6out[r]);
   }
-  Q1Requests rq = q1_one(q1[0], q1out[0], q1status[0]);
-  if (n1 == 2) {
-    const int lo = q1[1].ship_le < q1[0].ship_le ? 1 : 0;
-    for (int j = 0; j < 2; j++) {
-      const int r = j ? 1 - lo : lo;
-      rq.cut[j] = q1[r].ship_le;
-      rq.out[j] = static_cast<u128*>(q1out[r]);
-      rq.status[j] = q1status[r];
-    }
+  if (n1 == 1) return launch_q1_smem(call, c, q1_one(q1[0], q1out[0], q1status[0]), kRiding[n6], rd);
+  Q1Requests<2> rq;
+  const int lo = q1[1].ship_le < q1[0].ship_le ? 1 : 0;
+  for (int j = 0; j < 2; j++) {
+    const int r = j ? 1 - lo : lo;
+    rq.cut[j] = q1[r].ship_le;
+    rq.out[j] = static_cast<u128*>(q1out[r]);
+    rq.status[j] = q1status[r];
   }
-  return launch_q1_smem(call, c, rq, n1, kRiding[n1 - 1][n6], rd);
+  return launch_q1_smem(call, c, rq, kRiding2[n6], rd);
 }
 
 }  // namespace gpudb
@@ -1060,7 +1068,7 @@ extern "C" int gpudb_q1_group6(gpudb_ctx* ctx, const gpudb_lineitem* li, const g
   if ((rc = direct ? call.begin_direct(bytes) : call.begin(bytes))) return rc;
   const gpudb_q1_params pp = *p;
   if (uint8_t* d = call.direct_slot()) {
-    rc = launch_q1_smem(call, *li, q1_one(pp, d + kSlotHeader, nullptr), 1, q1_smem_kernel(variant), Q6Riders{},
+    rc = launch_q1_smem(call, *li, q1_one(pp, d + kSlotHeader, nullptr), q1_smem_kernel(variant), Q6Riders{},
                         reinterpret_cast<uint32_t*>(d));
   } else {
     void* dout = call.result<void>();
