@@ -172,7 +172,7 @@ constexpr uint32_t kQ13StageBytes = 32 * (GPUDB_COMMENT_WIDTH + 4);
 
 struct Q13Smem {
   unsigned char stage[kQ13Warps][kQ13Stages][kQ13StageBytes];   // 32 slots, then 32 customer keys
-  uint2 queue[kQ13Warps][64];                                   // {row, customer}
+  uint2 queue[kQ13Warps][64];                                   // {the warp's step * 32 + lane, customer}
   uint64_t full[kQ13Warps][kQ13Stages];
   __align__(4) uint8_t w[2][16];
 };
@@ -210,7 +210,10 @@ __global__ void __launch_bounds__(kQ13Threads, LONG ? 4 : 3) q13_count_kernel(co
       if (t0 + q * W < whole) issue(t0 + q * W, q);
   uint32_t queued = 0, parity = 0;
   int q = 0;
-  for (uint64_t t = t0;; t += W) {
+  // The queue names an order by the warp's step and the lane: 32 bits of it last for any row
+  // count, 32 bits of the row would not.
+  uint32_t step = 0;
+  for (uint64_t t = t0;; t += W, step++) {
     const bool more = t < tiles;
     if (more) {
       const uint64_t r = t * 32 + lane;
@@ -242,7 +245,7 @@ __global__ void __launch_bounds__(kQ13Threads, LONG ? 4 : 3) q13_count_kernel(co
       const bool maybe = known && may_hold<LONG>(rw, pat);
       if (known && !maybe) atomicAdd(counts + c, 1u);
       const uint32_t m = __ballot_sync(FULL_MASK, maybe);
-      if (maybe) queue[queued + __popc(m & lanemask_lt())] = make_uint2((uint32_t)r, (uint32_t)c);
+      if (maybe) queue[queued + __popc(m & lanemask_lt())] = make_uint2(step * 32 + lane, (uint32_t)c);
       queued += __popc(m);
       __syncwarp();
     }
@@ -251,7 +254,8 @@ __global__ void __launch_bounds__(kQ13Threads, LONG ? 4 : 3) q13_count_kernel(co
       queued -= take;
       if ((uint32_t)lane < take) {
         const uint2 e = queue[queued + lane];
-        const uint8_t* row = text + (uint64_t)e.x * GPUDB_COMMENT_WIDTH;
+        const uint64_t r = (t0 + (uint64_t)(e.x >> 5) * W) * 32 + (e.x & 31u);
+        const uint8_t* row = text + r * GPUDB_COMMENT_WIDTH;
         uint32_t rw[kSlotWords];
         load_slot(row, vec, rw);
         if (!like2<LONG>(rw, row, vec, pat, S.w)) atomicAdd(counts + e.y, 1u);

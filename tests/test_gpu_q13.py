@@ -2,6 +2,8 @@
 other word pairs, hand-written comments at the pattern's edge cases (adjacent words, words
 in the wrong order, a word cut by the 80-byte slot end, one-letter words, empty comments),
 customers without orders, orders of unknown customers, and the count and word limits."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -97,3 +99,85 @@ def test_q13_tiles_and_candidates(engine, orc, n_or, w1, w2):
     od = dict(cust_key=rng.integers(-1, 1001, n_or).astype(np.int32), comment=pool[rng.integers(0, len(pool), n_or)])
     cu = dict(cust_key=np.arange(1000, dtype=np.int32))
     assert run(engine, cu, od, w1, w2) == orc.q13(cu, od, w1, w2)
+
+
+class _Repeated:
+    """An address range of `size` bytes over `chunk` bytes of memory mapped again and again, its last
+    `tail` bytes over memory of their own."""
+
+    class _Prop(C.Structure):
+        _fields_ = [("type", C.c_int), ("handle", C.c_int), ("loc", C.c_int * 2), ("win32", C.c_void_p),
+                    ("flags", C.c_uint8 * 8)]
+
+    class _Access(C.Structure):
+        _fields_ = [("loc", C.c_int * 2), ("flags", C.c_int)]
+
+    def __init__(self, size, chunk, tail):
+        self.cu = C.CDLL("libcuda.so.1")
+        self.size, self.maps, self.handles, self.va = size, [], [], C.c_uint64(0)
+        assert (size - tail) % chunk == 0
+        self.check("cuMemAddressReserve", C.byref(self.va), C.c_size_t(size), C.c_size_t(0), C.c_uint64(0), C.c_ulonglong(0))
+        body, end = self.alloc(chunk), self.alloc(tail)
+        for at in range(0, size - tail, chunk):
+            self.map(at, chunk, body)
+        self.map(size - tail, tail, end)
+        acc = self._Access((C.c_int * 2)(1, 0), 3)   # device 0, read and write
+        self.check("cuMemSetAccess", self.va, C.c_size_t(size), C.byref(acc), C.c_size_t(1))
+
+    def check(self, name, *args):
+        rc = getattr(self.cu, name)(*args)
+        assert rc == 0, (name, rc)
+
+    def alloc(self, size):
+        prop = self._Prop(type=1, loc=(C.c_int * 2)(1, 0))   # pinned, device 0
+        h = C.c_uint64(0)
+        self.check("cuMemCreate", C.byref(h), C.c_size_t(size), C.byref(prop), C.c_ulonglong(0))
+        self.handles.append(h)
+        return h
+
+    def map(self, at, size, handle):
+        self.check("cuMemMap", C.c_uint64(self.va.value + at), C.c_size_t(size), C.c_size_t(0), handle, C.c_ulonglong(0))
+        self.maps.append((at, size))
+
+    def close(self):
+        for at, size in self.maps:
+            self.check("cuMemUnmap", C.c_uint64(self.va.value + at), C.c_size_t(size))
+        for h in self.handles:
+            self.check("cuMemRelease", h)
+        self.check("cuMemAddressFree", self.va, C.c_size_t(self.size))
+
+
+def test_q13_more_than_2_to_the_32_orders(engine, orc):
+    """Orders from row 2^32 on are matched with their own comments (344 GB of comments, the first 2^32
+    of them one block of memory mapped 512 times: no comment, no known customer)."""
+    head, tail, period = 1 << 32, 1 << 19, 1 << 23
+    text = _Repeated((head + tail) * 80, period * 80, tail * 80)
+    cust = _Repeated((head + tail) * 4, period * 4, tail * 4)
+    try:
+        zeros, none = np.zeros(period * 80, np.uint8), np.full(period, -1, np.int32)
+        comments = np.where(np.arange(tail) % 3 == 0, np.array(b"special requests", "S80"),
+                            np.array(b"special packages", "S80")).astype("S80")
+        ck = (np.arange(tail) % 1000).astype(np.int32)
+        for dst, src in ((text.va.value, zeros), (text.va.value + head * 80, comments),
+                         (cust.va.value, none), (cust.va.value + head * 4, ck)):
+            engine._check(engine.lib.gpudb_copy(engine.ctx, dst, src.ctypes.data, src.nbytes))
+        cu = dict(cust_key=np.arange(1000, dtype=np.int32))
+        tc = engine.upload("customer", cu)
+        got = engine.q13(tc, _View(capi.Orders(n_rows=head + tail, cust_key=cust.va.value, comment=text.va.value,
+                                               key_max=-1, cust_key_max=999)))
+        engine.free(tc)
+        assert got == orc.q13(cu, dict(cust_key=ck, comment=comments))
+    finally:
+        engine.sync()
+        text.close()
+        cust.close()
+
+
+class _View:
+    """A table given as its C struct."""
+
+    def __init__(self, s):
+        self.s = s
+
+    def struct(self):
+        return self.s
