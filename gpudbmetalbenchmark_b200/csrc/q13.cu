@@ -64,6 +64,67 @@ __device__ __forceinline__ bool word_at(const uint8_t* row, bool vec, int pos, c
   return true;
 }
 
+// How the orders are tested, from the words' lengths:
+//  kLong    both words of kLongWord letters or more (see candidates): queue the orders that may hold w0;
+//  kBytes   w0 of three letters or more: the same with a compare at every byte;
+//  kDirect  w0 of one or two letters, which most comments hold: a queue of nearly every order costs
+//           more than it saves, so every order is matched at once (like2_short). 15M orders, whole
+//           call: "s", "s" 332 us, queued 750; "ar", "ar" 517 us, queued 482 (few orders hold it);
+//           "s ", " s" 504 us, queued 698.
+enum Q13Form { kLong, kBytes, kDirect };
+
+// High bit of every byte of x that is zero (exact per byte).
+__device__ __forceinline__ uint32_t zero_bytes(uint32_t x) {
+  const uint32_t y = (x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu;
+  return ~(y | x | 0x7F7F7F7Fu);
+}
+
+// The positions of a row whose first two bytes (one letter: first byte) are those of word `w`:
+// SWAR on the row word and the row word shifted by one byte. The flags of word k (bits 7, 15, 23,
+// 31) land on bits (k & 7) + {0, 8, 16, 24} of c[k >> 3].
+__device__ __forceinline__ void pair_flags(const uint32_t (&rw)[kSlotWords], const Q13Pattern& pat, int w, uint32_t (&c)[3]) {
+  const uint32_t a = pat.w[w][0] * 0x01010101u, b = pat.w[w][1] * 0x01010101u;
+  c[0] = c[1] = c[2] = 0;
+  auto mark = [&](int k, uint32_t m) { c[k >> 3] |= (m >> (7 - (k & 7))) & (0x01010101u << (k & 7)); };
+  if (pat.len[w] == 1) {
+#pragma unroll
+    for (int k = 0; k < kSlotWords; k++) mark(k, zero_bytes(rw[k] ^ a));
+  } else {
+#pragma unroll
+    for (int k = 0; k < kSlotWords; k++) {
+      const uint32_t x = rw[k], nx = k + 1 < kSlotWords ? rw[k + 1] : 0u;
+      mark(k, zero_bytes(x ^ a) & zero_bytes(__funnelshift_r(x, nx, 8) ^ b));
+    }
+  }
+}
+
+// LIKE '%w0%w1%' on a row per lane, w0 of at most two letters, so that its flags are all of it and
+// the first one decides; the positions of a longer w1 behind it are compared in full. Every lane
+// of the warp calls it; w1 is not looked for when none of them has a w0.
+__device__ __forceinline__ bool like2_short(const uint32_t (&rw)[kSlotWords], const uint8_t* row, bool vec, bool known,
+                                            const Q13Pattern& pat, const uint8_t (&w)[2][16]) {
+  uint32_t c0[3], c1[3];
+  pair_flags(rw, pat, 0, c0);
+  const int q = c0[0] ? 0 : c0[1] ? 1 : 2;
+  const uint32_t c = q == 0 ? c0[0] : q == 1 ? c0[1] : c0[2];
+  if (!__any_sync(FULL_MASK, known && c)) return false;
+  pair_flags(rw, pat, 1, c1);
+  if (!known || !c) return false;
+  const int j = __ffs((c | c >> 8 | c >> 16 | c >> 24) & 0xFFu) - 1;   // the first word with a w0
+  const int l1 = pat.len[1], start = 4 * (8 * q + j) + ((__ffs((c >> j) & 0x01010101u) - 1) >> 3) + pat.len[0];
+#pragma unroll
+  for (int q1 = 2; q1 >= 0; q1--) {
+    uint32_t m = c1[q1];
+    while (m) {
+      const int b = __ffs(m) - 1;
+      m &= m - 1;
+      const int pos = 4 * (8 * q1 + (b & 7)) + (b >> 3);
+      if (pos >= start && (l1 <= 2 || word_at(row, vec, pos, w[1], l1))) return true;
+    }
+  }
+  return false;
+}
+
 // Calls f(hit, position) for the places where a word may start; every place where it does
 // start has a hit. LONG: a word of 7 letters or more covers a whole aligned 32-bit word of the
 // row wherever it starts, so each row word is compared with the four words that can stand
@@ -86,8 +147,9 @@ __device__ __forceinline__ void candidates(const uint32_t (&rw)[kSlotWords], con
 
 // Whether the row may hold word 0. The LONG compares run on the half-rate integer pipe and
 // bind the kernel, so every other row word takes the polynomial instead, whose four multiplies
-// run on the multiply pipe: it is 0 where the word equals one of the four (and for about one
-// other word in a million, which the full match turns away).
+// run on the multiply pipe: it is 0 where the word equals one of the four, and for the few other
+// words whose differences from the four multiply to 0 mod 2^32, which the full match turns away
+// (more of them for a w0 that repeats letters: "aaaaaaa" 293 us a call, "special" 290).
 template <bool LONG>
 __device__ __forceinline__ bool may_hold(const uint32_t (&rw)[kSlotWords], const Q13Pattern& pat) {
   bool any = false;
@@ -177,8 +239,8 @@ struct Q13Smem {
   __align__(4) uint8_t w[2][16];
 };
 
-template <bool LONG>
-__global__ void __launch_bounds__(kQ13Threads, LONG ? 4 : 3) q13_count_kernel(const char* __restrict__ comment,
+template <Q13Form FORM>
+__global__ void __launch_bounds__(kQ13Threads, FORM != kBytes ? 4 : 3) q13_count_kernel(const char* __restrict__ comment,
                                                                     const int32_t* __restrict__ ocust, uint64_t n,
                                                                     int32_t cust_max,
                                                                     const __grid_constant__ Q13Pattern pat,
@@ -218,7 +280,7 @@ __global__ void __launch_bounds__(kQ13Threads, LONG ? 4 : 3) q13_count_kernel(co
     if (more) {
       const uint64_t r = t * 32 + lane;
       const bool in = r < n;
-      uint32_t rw[kSlotWords];
+      uint32_t rw[kSlotWords] = {};
       int32_t c = -1;
       if (t < whole) {
         if (!__all_sync(FULL_MASK, mbar_wait(&S.full[warp][q], parity, kMbarPollLimit))) {
@@ -242,7 +304,12 @@ __global__ void __launch_bounds__(kQ13Threads, LONG ? 4 : 3) q13_count_kernel(co
         load_slot(text + r * GPUDB_COMMENT_WIDTH, vec, rw);
       }
       const bool known = in && c >= 0 && c <= cust_max;   // an order of no known customer counts for nobody
-      const bool maybe = known && may_hold<LONG>(rw, pat);
+      if (FORM == kDirect) {
+        if (!like2_short(rw, text + r * GPUDB_COMMENT_WIDTH, vec, known, pat, S.w) && known) atomicAdd(counts + c, 1u);
+        __syncwarp();
+        continue;
+      }
+      const bool maybe = known && may_hold<FORM == kLong>(rw, pat);
       if (known && !maybe) atomicAdd(counts + c, 1u);
       const uint32_t m = __ballot_sync(FULL_MASK, maybe);
       if (maybe) queue[queued + __popc(m & lanemask_lt())] = make_uint2(step * 32 + lane, (uint32_t)c);
@@ -258,7 +325,7 @@ __global__ void __launch_bounds__(kQ13Threads, LONG ? 4 : 3) q13_count_kernel(co
         const uint8_t* row = text + r * GPUDB_COMMENT_WIDTH;
         uint32_t rw[kSlotWords];
         load_slot(row, vec, rw);
-        if (!like2<LONG>(rw, row, vec, pat, S.w)) atomicAdd(counts + e.y, 1u);
+        if (!like2<FORM == kLong>(rw, row, vec, pat, S.w)) atomicAdd(counts + e.y, 1u);
       }
       __syncwarp();
     }
@@ -334,7 +401,6 @@ extern "C" int gpudb_q13_distribution(gpudb_ctx* ctx, const gpudb_customer* cu, 
   c[2] = q01 + q23 + s01 * s23;
   c[1] = s01 * q23 + s23 * q01;
   c[0] = q01 * q23;
-  const bool long_words = pat.len[0] >= kLongWord && pat.len[1] >= kLongWord;
   Call call(ctx, ex, t);
   const size_t bytes = 16 + (size_t)kBins * sizeof(gpudb_q13_row);
   int rc = call.begin(bytes, true);
@@ -348,7 +414,9 @@ extern "C" int gpudb_q13_distribution(gpudb_ctx* ctx, const gpudb_customer* cu, 
   if ((rc = call.clear(hist, 0, (size_t)kBins * 4))) return rc;
   const int sms = ctx->sm_count;
   if (od->n_rows && cu->n_rows) {
-    auto kern = long_words ? q13_count_kernel<true> : q13_count_kernel<false>;
+    auto kern = pat.len[0] <= 2                                          ? q13_count_kernel<kDirect>
+                : pat.len[0] >= kLongWord && pat.len[1] >= kLongWord ? q13_count_kernel<kLong>
+                                                                     : q13_count_kernel<kBytes>;
     GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)kern, sizeof(Q13Smem)));
     const int per_sm = kernel_occupancy(ctx, (const void*)kern, kQ13Threads, sizeof(Q13Smem));
     const unsigned g = (unsigned)std::max<uint64_t>(

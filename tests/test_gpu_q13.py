@@ -181,3 +181,23 @@ class _View:
 
     def struct(self):
         return self.s
+
+
+@pytest.mark.parametrize("w1,w2", [(b"a", b"a"), (b"q", b"zz"), (b"ab", b"ba"), (b"aa", b"a"), (b"zz", b"special"),
+                                   (b"a", b"aaaaaaaaaaaaaaa")])
+def test_q13_first_word_of_one_or_two_letters(engine, orc, w1, w2):
+    """Such orders are matched without a queue: the words at every pair of places, next to each
+    other and overlapping, at the ends of the slot, and comments without the first word."""
+    rng = np.random.default_rng(len(w1) * 16 + len(w2))
+    texts = [b"", b"b" * 79, w1, w2, w2 + w1, w1 + w2, w1[:1] * 79, w2[:1] * 80]
+    for at in range(80 - len(w1) + 1):
+        for gap in (0, 1, 2, 3, 7, 40):
+            t = b"-" * at + w1 + b"-" * gap + w2
+            texts += [t[:80], t[:79], (b"-" * at + w1)[:80]]
+        texts.append((w2 + b"-" * at + w1)[:80])
+    alphabet = np.frombuffer(w1 + w2 + b"- ", np.uint8)
+    texts += [bytes(rng.choice(alphabet, int(rng.integers(0, 81)))) for _ in range(3000)]
+    n = len(texts)
+    od = dict(cust_key=rng.integers(-1, 301, n).astype(np.int32), comment=np.array(texts, dtype="S80"))
+    cu = dict(cust_key=np.arange(300, dtype=np.int32))
+    assert run(engine, cu, od, w1, w2) == orc.q13(cu, od, w1, w2)
