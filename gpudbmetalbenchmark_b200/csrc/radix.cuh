@@ -119,6 +119,10 @@ __global__ void __launch_bounds__(kRxThreads) rx_hist_kernel(ColumnSource<P> src
   const uint64_t super_rows = rx_super_rows_for(n, G, tile);
   const uint64_t r0 = (uint64_t)blockIdx.x * super_rows;
   const uint32_t rows = r0 < n ? (uint32_t)min(super_rows, n - r0) : 0u;
+  if (F == 1) {   // one digit: the rows need no reading
+    if (threadIdx.x == 0) hist[blockIdx.x] = rows;
+    return;
+  }
   const int32_t* keys = src.keys + r0;
   auto add = [&](int32_t k, uint32_t run) {
     const uint32_t h = key_hash32(k);
@@ -137,8 +141,10 @@ __global__ void __launch_bounds__(kRxThreads) rx_hist_kernel(ColumnSource<P> src
     add(k.w, run);
   };
   constexpr uint32_t U = 4;   // quads in flight per thread
-  const uint32_t quads = ((uintptr_t)keys & 15u) == 0 ? rows / 4 : 0;
-  const int4* keys4 = reinterpret_cast<const int4*>(keys);
+  // the rows before the first 16-byte boundary, then quads, then the rest
+  const uint32_t lead = min(rows, (uint32_t)(0u - ((uintptr_t)keys >> 2)) & 3u), quads = (rows - lead) / 4;
+  const int4* keys4 = reinterpret_cast<const int4*>(keys + lead);
+  if (threadIdx.x < lead) add(__ldg(keys + threadIdx.x), 1u);
   uint32_t q = threadIdx.x;
   for (; q + (U - 1) * kRxThreads < quads; q += U * kRxThreads) {
     int4 k[U];
@@ -148,7 +154,8 @@ __global__ void __launch_bounds__(kRxThreads) rx_hist_kernel(ColumnSource<P> src
     for (uint32_t u = 0; u < U; u++) quad(k[u]);
   }
   for (; q < quads; q += kRxThreads) quad(__ldg(keys4 + q));
-  for (uint32_t i = quads * 4 + threadIdx.x; i < rows; i += kRxThreads) add(__ldg(keys + i), 1u);
+  const uint32_t rest = lead + quads * 4 + threadIdx.x;
+  if (rest < rows) add(__ldg(keys + rest), 1u);
   __syncthreads();
   for (uint32_t b = threadIdx.x; b < F; b += kRxThreads) hist[(size_t)b * G + blockIdx.x] = cnt[b];
   if (fs)

@@ -208,6 +208,27 @@ def test_join_count_direct_edges(engine, orc):
         engine.device_free(dq)
 
 
+@pytest.mark.parametrize("bits", [0, 1, 8, 13])
+@pytest.mark.parametrize("first", [1, 2, 3])
+def test_radix_partition_columns_off_16_bytes(engine, orc, bits, first):
+    """Keys and payload that start `first` rows off a 16-byte boundary: fewer rows than up to the
+    boundary, up to it, one past it, and many sub-tiles; clustered keys and one key alone."""
+    for n in (1, 2, 3, 4, 5, 8193, 400_009):
+        for keys in (orc.gen(8, n + first, seed=n, n_orders=max(n // 3, 1), order_mode=1), np.full(n + first, 77, np.int32)):
+            pay = np.arange(n + first, dtype=np.int32) * 5
+            dk, dp = engine.to_device(keys), engine.to_device(pay)
+            ko, po, off = (engine.device_array(n * 4), engine.device_array(n * 4), engine.device_array(((1 << bits) + 1) * 4))
+            try:
+                engine.radix_partition(dk + 4 * first, dp + 4 * first, n, bits, ko, po, off)
+                wk, wp, woff = orc.radix_partition(keys[first:], pay[first:], bits)
+                assert np.array_equal(engine.to_host(off, (1 << bits) + 1, np.uint32), woff)
+                assert np.array_equal(engine.to_host(ko, n, np.int32), wk)
+                assert np.array_equal(engine.to_host(po, n, np.int32), wp)
+            finally:
+                for x in (dk, dp, ko, po, off):
+                    engine.device_free(x)
+
+
 def test_radix_partition_bad_bits(engine):
     with pytest.raises(capi.GpudbError) as e:
         engine.radix_partition(None, None, 0, 17, 1, 1, 1)
