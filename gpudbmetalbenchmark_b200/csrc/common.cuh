@@ -87,13 +87,19 @@ __device__ __forceinline__ bool bitmap_test(const uint32_t* bm, int32_t key) {
 // ---- streaming loads (read once: do not keep in L1) ---------------------------------------
 template <class T> __device__ __forceinline__ T ld_stream(const T* p) { return __ldcs(p); }
 
-// Four consecutive rows i .. i + 3 of a column of n (i a multiple of 4): one 16-byte load (two
-// for 8-byte values, one of 4 for bytes) where the column's start allows it and the rows are
-// all there, else one load a row; `fill` past the end. A warp then reads 512 consecutive bytes
-// of a 4-byte column with one instruction, and rows of one order sit in one thread.
+// Four consecutive rows i .. i + 3 of a column of n (i a multiple of 4) that starts on 16 bytes (bytes:
+// on 4): one load where the rows are all there, else one a row; `fill` past the end. A warp then
+// reads 512 consecutive bytes of a 4-byte column with one instruction, and rows of one order sit
+// in one thread. Columns that start elsewhere are for rows strided over the block: loaded so, each
+// of a thread's four loads would spread a warp over four times the lines.
+inline bool quad_start(const int32_t* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline bool quad_start(const uint8_t* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }
+template <class... P>
+bool rows4_ok(const P*... cols) { return (quad_start(cols) && ...); }
+
 __device__ __forceinline__ void ld_rows4(const int32_t* __restrict__ col, uint64_t i, uint64_t n, int32_t fill,
                                          int32_t (&o)[4]) {
-  if ((reinterpret_cast<uintptr_t>(col) & 15u) == 0 && i + 4 <= n) {
+  if (i + 4 <= n) {
     const int4 v = ld_stream(reinterpret_cast<const int4*>(col + i));
     o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
   } else {
@@ -103,7 +109,7 @@ __device__ __forceinline__ void ld_rows4(const int32_t* __restrict__ col, uint64
 }
 __device__ __forceinline__ void ld_rows4(const uint8_t* __restrict__ col, uint64_t i, uint64_t n, uint32_t fill,
                                          uint32_t (&o)[4]) {
-  if ((reinterpret_cast<uintptr_t>(col) & 3u) == 0 && i + 4 <= n) {
+  if (i + 4 <= n) {
     const uint32_t v = ld_stream(reinterpret_cast<const uint32_t*>(col + i));
     o[0] = v & 0xFFu; o[1] = (v >> 8) & 0xFFu; o[2] = (v >> 16) & 0xFFu; o[3] = v >> 24;
   } else {

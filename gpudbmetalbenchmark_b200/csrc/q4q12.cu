@@ -24,7 +24,7 @@ namespace gpudb {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kRows = 4;   // consecutive rows per thread per block step (ld_rows4)
+constexpr int kRows = 4;   // rows per thread per block step: consecutive (QUAD, ld_rows4) or strided over the block
 
 // Adds the block's per-thread bins into out[0..B) (one atomic per nonzero bin per block).
 template <int B>
@@ -47,6 +47,7 @@ __device__ __forceinline__ void block_add_bins(const uint32_t (&c)[B], unsigned 
 // consecutive rows a thread, so that most of a bitmap word's rows merge in registers: one warp
 // merge per 128 rows instead of four (Q4 and Q12 over 50M rows: 386 us a pair of calls with rows
 // strided over the block, 344 us here; 6M rows: 112 and 107 us).
+template <bool QUAD>
 __global__ void __launch_bounds__(kThreads) q4_late_kernel(const int32_t* __restrict__ key,
                                                            const int32_t* __restrict__ commit,
                                                            const int32_t* __restrict__ receipt, uint64_t n,
@@ -54,19 +55,35 @@ __global__ void __launch_bounds__(kThreads) q4_late_kernel(const int32_t* __rest
   const uint64_t step = (uint64_t)gridDim.x * kThreads * kRows;
   for (uint64_t b = (uint64_t)blockIdx.x * kThreads * kRows; b < n; b += step) {   // whole warps
     int32_t k[kRows], c[kRows], r[kRows];
-    const uint64_t i0 = b + 4 * threadIdx.x;
-    ld_rows4(key, i0, n, -1, k);
-    ld_rows4(commit, i0, n, 0, c);
-    ld_rows4(receipt, i0, n, 0, r);
+    if (QUAD) {
+      const uint64_t i0 = b + 4 * threadIdx.x;
+      ld_rows4(key, i0, n, -1, k);
+      ld_rows4(commit, i0, n, 0, c);
+      ld_rows4(receipt, i0, n, 0, r);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kRows; j++) {
+        const uint64_t i = b + (uint64_t)j * kThreads + threadIdx.x;
+        const bool in = i < n;
+        k[j] = in ? ld_stream(key + i) : -1;
+        c[j] = in ? ld_stream(commit + i) : 0;
+        r[j] = in ? ld_stream(receipt + i) : 0;
+      }
+    }
     uint32_t on = 0;
 #pragma unroll
-    for (int j = 0; j < kRows; j++) on |= (uint32_t)(c[j] < r[j] && k[j] >= 0 && k[j] <= key_max) << j;
-    warp_bitmap_or4(on, k, bits);
+    for (int j = 0; j < kRows; j++) {
+      const bool late = c[j] < r[j] && k[j] >= 0 && k[j] <= key_max;
+      if (QUAD) on |= (uint32_t)late << j;
+      else warp_bitmap_or(late, k[j], bits);
+    }
+    if (QUAD) warp_bitmap_or4(on, k, bits);
   }
 }
 
 // Orders in [date_lo, date_hi) whose key is in the late bitmap, counted by priority 1..5
 // (kernels/q4.metal:40-72). An order key outside 0..key_max is a key-range error.
+template <bool QUAD>
 __global__ void __launch_bounds__(kThreads) q4_count_kernel(const int32_t* __restrict__ okey,
                                                             const int32_t* __restrict__ odate,
                                                             const uint8_t* __restrict__ oprio, uint64_t n,
@@ -78,10 +95,21 @@ __global__ void __launch_bounds__(kThreads) q4_count_kernel(const int32_t* __res
   for (uint64_t b = (uint64_t)blockIdx.x * kThreads * kRows; b < n; b += step) {
     int32_t k[kRows], d[kRows];
     uint32_t p[kRows];
-    const uint64_t i0 = b + 4 * threadIdx.x;
-    ld_rows4(odate, i0, n, date_hi, d);
-    ld_rows4(okey, i0, n, 0, k);
-    ld_rows4(oprio, i0, n, 0u, p);
+    if (QUAD) {
+      const uint64_t i0 = b + 4 * threadIdx.x;
+      ld_rows4(odate, i0, n, date_hi, d);
+      ld_rows4(okey, i0, n, 0, k);
+      ld_rows4(oprio, i0, n, 0u, p);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kRows; j++) {
+        const uint64_t i = b + (uint64_t)j * kThreads + threadIdx.x;
+        const bool in = i < n;
+        d[j] = in ? ld_stream(odate + i) : date_hi;
+        k[j] = in ? ld_stream(okey + i) : 0;
+        p[j] = in ? ld_stream(oprio + i) : 0u;
+      }
+    }
 #pragma unroll
     for (int j = 0; j < kRows; j++) {
       if (d[j] < date_lo || d[j] >= date_hi) continue;
@@ -96,6 +124,7 @@ __global__ void __launch_bounds__(kThreads) q4_count_kernel(const int32_t* __res
 
 // ---- Q12 -----------------------------------------------------------------------------------
 // Priority bitmap (kernels/q12.metal:87-99): orders with priority 1..high_max.
+template <bool QUAD>
 __global__ void __launch_bounds__(kThreads) q12_prio_kernel(const int32_t* __restrict__ okey,
                                                             const uint8_t* __restrict__ oprio, uint64_t n,
                                                             int32_t high_max, int32_t key_max, uint32_t* bits,
@@ -104,17 +133,28 @@ __global__ void __launch_bounds__(kThreads) q12_prio_kernel(const int32_t* __res
   for (uint64_t b = (uint64_t)blockIdx.x * kThreads * kRows; b < n; b += step) {   // whole warps
     int32_t k[kRows];
     uint32_t p[kRows];
-    const uint64_t i0 = b + 4 * threadIdx.x;
-    ld_rows4(okey, i0, n, 0, k);
-    ld_rows4(oprio, i0, n, 0u, p);
+    if (QUAD) {
+      const uint64_t i0 = b + 4 * threadIdx.x;
+      ld_rows4(okey, i0, n, 0, k);
+      ld_rows4(oprio, i0, n, 0u, p);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kRows; j++) {
+        const uint64_t i = b + (uint64_t)j * kThreads + threadIdx.x;
+        const bool in = i < n;
+        k[j] = in ? ld_stream(okey + i) : 0;
+        p[j] = in ? ld_stream(oprio + i) : 0u;
+      }
+    }
     uint32_t set = 0;
 #pragma unroll
     for (int j = 0; j < kRows; j++) {
       bool on = p[j] >= 1u && p[j] <= (uint32_t)high_max;
       if (on && (k[j] < 0 || k[j] > key_max)) { set_status(status, ST_KEY_RANGE); on = false; }
-      set |= (uint32_t)on << j;
+      if (QUAD) set |= (uint32_t)on << j;
+      else warp_bitmap_or(on, k[j], bits);
     }
-    warp_bitmap_or4(set, k, bits);
+    if (QUAD) warp_bitmap_or4(set, k, bits);
   }
 }
 
@@ -125,6 +165,7 @@ struct Q12Args {
 // Lineitem rows of ship mode mode0 / mode1 with receipt in [lo, hi), commit < receipt and
 // ship < commit, counted high or low by the priority bitmap (kernels/q12.metal:22-66).
 // Bins: out[0..1] high for mode0/mode1, out[2..3] low.
+template <bool QUAD>
 __global__ void __launch_bounds__(kThreads) q12_count_kernel(const int32_t* __restrict__ lkey,
                                                              const int32_t* __restrict__ lship,
                                                              const int32_t* __restrict__ lcommit,
@@ -137,12 +178,25 @@ __global__ void __launch_bounds__(kThreads) q12_count_kernel(const int32_t* __re
   for (uint64_t b = (uint64_t)blockIdx.x * kThreads * kRows; b < n; b += step) {
     int32_t k[kRows], s[kRows], c[kRows], r[kRows];
     uint32_t m[kRows];
-    const uint64_t i0 = b + 4 * threadIdx.x;
-    ld_rows4(lmode, i0, n, ~0u, m);
-    ld_rows4(lreceipt, i0, n, 0, r);
-    ld_rows4(lcommit, i0, n, 0, c);
-    ld_rows4(lship, i0, n, 0, s);
-    ld_rows4(lkey, i0, n, -1, k);
+    if (QUAD) {
+      const uint64_t i0 = b + 4 * threadIdx.x;
+      ld_rows4(lmode, i0, n, ~0u, m);
+      ld_rows4(lreceipt, i0, n, 0, r);
+      ld_rows4(lcommit, i0, n, 0, c);
+      ld_rows4(lship, i0, n, 0, s);
+      ld_rows4(lkey, i0, n, -1, k);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kRows; j++) {
+        const uint64_t i = b + (uint64_t)j * kThreads + threadIdx.x;
+        const bool in = i < n;
+        m[j] = in ? ld_stream(lmode + i) : ~0u;
+        r[j] = in ? ld_stream(lreceipt + i) : 0;
+        c[j] = in ? ld_stream(lcommit + i) : 0;
+        s[j] = in ? ld_stream(lship + i) : 0;
+        k[j] = in ? ld_stream(lkey + i) : -1;
+      }
+    }
 #pragma unroll
     for (int j = 0; j < kRows; j++) {
       const int mi = (int32_t)m[j] == a.mode0 ? 0 : ((int32_t)m[j] == a.mode1 ? 1 : -1);
@@ -192,12 +246,14 @@ extern "C" int gpudb_q4_priority(gpudb_ctx* ctx, const gpudb_orders* od, const g
   if (od->n_rows) {
     rc = stream_lineitem(call, li, mask, 0, [&](const gpudb_lineitem& c) {
       if (c.n_rows)
-        GPUDB_LAUNCH(call, q4_late_kernel, scan_grid(ctx, c.n_rows), kThreads, 0, c.order_key, c.commit_date,
+        GPUDB_LAUNCH(call, (rows4_ok(c.order_key, c.commit_date, c.receipt_date) ? q4_late_kernel<true> : q4_late_kernel<false>),
+                 scan_grid(ctx, c.n_rows), kThreads, 0, c.order_key, c.commit_date,
                      c.receipt_date, c.n_rows, key_max, (uint32_t*)bits);
       return (int)GPUDB_OK;
     });
     if (rc) return rc;
-    GPUDB_LAUNCH(call, q4_count_kernel, scan_grid(ctx, od->n_rows), kThreads, 0, od->order_key, od->order_date,
+    GPUDB_LAUNCH(call, (rows4_ok(od->order_key, od->order_date, od->priority) ? q4_count_kernel<true> : q4_count_kernel<false>),
+                 scan_grid(ctx, od->n_rows), kThreads, 0, od->order_key, od->order_date,
                  od->priority, od->n_rows, p->date_lo, p->date_hi, key_max, (const uint32_t*)bits,
                  call.result<unsigned long long>(), call.status());
   }
@@ -225,13 +281,15 @@ extern "C" int gpudb_q12_shipmode(gpudb_ctx* ctx, const gpudb_orders* od, const 
   if ((rc = scratch(ctx, "q12.high", (size_t)words * 4, &bits))) return rc;
   if ((rc = call.clear(bits, 0, (size_t)words * 4))) return rc;
   if (od->n_rows)
-    GPUDB_LAUNCH(call, q12_prio_kernel, scan_grid(ctx, od->n_rows), kThreads, 0, od->order_key, od->priority,
+    GPUDB_LAUNCH(call, (rows4_ok(od->order_key, od->priority) ? q12_prio_kernel<true> : q12_prio_kernel<false>),
+                 scan_grid(ctx, od->n_rows), kThreads, 0, od->order_key, od->priority,
                  od->n_rows, p->high_max, key_max, (uint32_t*)bits, call.status());
   // with no orders every row is low (an empty bitmap); its key bound is then -1
   const Q12Args a{p->receipt_lo, p->receipt_hi, p->mode[0], p->mode[1], od->n_rows ? key_max : -1};
   rc = stream_lineitem(call, li, mask, 0, [&](const gpudb_lineitem& c) {
     if (c.n_rows)
-      GPUDB_LAUNCH(call, q12_count_kernel, scan_grid(ctx, c.n_rows), kThreads, 0, c.order_key, c.ship_date,
+      GPUDB_LAUNCH(call, (rows4_ok(c.order_key, c.ship_date, c.commit_date, c.receipt_date, c.ship_mode) ? q12_count_kernel<true> : q12_count_kernel<false>),
+                 scan_grid(ctx, c.n_rows), kThreads, 0, c.order_key, c.ship_date,
                    c.commit_date, c.receipt_date, c.ship_mode, c.n_rows, a, (const uint32_t*)bits,
                    call.result<unsigned long long>());
     return (int)GPUDB_OK;

@@ -126,3 +126,40 @@ def test_missing_columns_are_rejected(engine, orc):
         assert e.value.code == capi.E_INVALID
     finally:
         free(engine, to, tl)
+
+
+class _View:
+    """A table given as its C struct."""
+
+    def __init__(self, s):
+        self.s = s
+
+    def struct(self):
+        return self.s
+
+
+@pytest.mark.parametrize("n_or,n_li,mode", [(30_001, 120_007, 1), (700, 2600, 2), (5, 7, 1)])
+@pytest.mark.parametrize("o_first,l_first,byte_off", [(0, 0, 0), (1, 1, 0), (0, 3, 0), (2, 0, 0), (0, 0, 1), (4, 4, 2)])
+def test_q4_q12_columns_off_16_bytes(engine, orc, n_or, n_li, mode, o_first, l_first, byte_off):
+    """Tables that begin some rows into their columns, and byte columns alone off their boundary:
+    rows strided over the block instead of four consecutive ones a thread."""
+    od, li = orc.q4_tables(n_or, n_li, 29, order_mode=mode)
+    to, tl = upload(engine, od, li)
+    so, sl = to.struct(), tl.lineitem(n_li - l_first, l_first)
+    so.n_rows = n_or - o_first
+    for name, width in (("order_key", 4), ("order_date", 4), ("priority", 1)):
+        setattr(so, name, getattr(so, name) + o_first * width)
+    extra = []
+    if byte_off:
+        for struct, name, col in ((so, "priority", od["priority"][o_first:]), (sl, "ship_mode", li["ship_mode"][l_first:])):
+            p = engine.to_device(np.concatenate([np.zeros(byte_off, np.uint8), col]))
+            extra.append(p)
+            setattr(struct, name, p + byte_off)
+    od2, li2 = {k: v[o_first:] for k, v in od.items()}, {k: v[l_first:] for k, v in li.items()}
+    try:
+        assert engine.q4(_View(so), sl, 0, 2600) == orc.q4(od2, li2, 0, 2600)
+        assert engine.q12(_View(so), sl, 0, 2600) == orc.q12(od2, li2, 0, 2600)
+    finally:
+        free(engine, to, tl)
+        for p in extra:
+            engine.device_free(p)
