@@ -202,3 +202,56 @@ def test_q3_radix_in_two_passes(engine, orc, bits):
     final partition stays contiguous): the result equals the oracle's."""
     cu, od, li = orc.q3_tables(3000, 20000, 80000, 5)
     assert run(engine, cu, od, li, capi.JOIN_RADIX, radix_bits=bits) == orc.q3(cu, od, li)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("first", [1, 2, 3])
+@pytest.mark.parametrize("n_li", [3, 130, 80_003])
+def test_q3_fact_columns_off_16_bytes(engine, orc, mode, first, n_li):
+    """A fact table that begins `first` rows into its columns: the row-at-a-time probes."""
+    cu, od, li = orc.q3_tables(3000, 20_000, n_li + first, 31)
+    tc, to, tl = engine.upload("customer", cu), engine.upload("orders", od), engine.upload("lineitem", li)
+    li2 = {k: v[first:] for k, v in li.items()}
+    try:
+        for d, s in ((1170, 1170), (2400, 100), (300, 2500)):
+            got = engine.q3(tc, to, tl.lineitem(n_li, first), order_date_lt=d, ship_date_gt=s, k=20, join_mode=mode)
+            assert got == orc.q3(cu, od, li2, 1, d, s, 20), (d, s)
+    finally:
+        for t in (tc, to, tl):
+            engine.free(t)
+
+
+@pytest.mark.parametrize("first", [0, 1])
+@pytest.mark.parametrize("key_max", [-1, 0, 12_001])
+def test_q3_global_order_keys_outside_the_bound(engine, orc, first, key_max):
+    """Order keys below 0 and above the declared bound turn the probe's order-key bitmap off: every
+    key is looked up in the table, -1 and the int32 extremes among them."""
+    cu, od, li = orc.q3_tables(3000, 20_000, 80_007, 41)
+    old = np.array([5, 9, 13, 17, 21, 25], np.int32)
+    new = np.array([-1, -7, 0, 2**31 - 1, -2**31 + 1, 2**30], np.int32)
+    od["order_date"][1:7] = 3
+    cu["segment"][od["cust_key"][1:7]] = 1
+    mine = np.isin(li["order_key"], old)
+    li["ship_date"][mine] = 2500
+    li["ext_price"][mine] += 100_000_000   # among the first of the answer
+    rows, groups = orc.q3(cu, od, {k: v[first:] for k, v in li.items()}, k=64)
+    to_new = dict(zip(old.tolist(), new.tolist()))
+    assert {r[0] for r in rows} >= set(old.tolist())
+    want = [(to_new.get(r[0], r[0]),) + tuple(r[1:]) for r in rows], groups
+    for t in (od, li):   # (the oracle's table is indexed by the key)
+        a = t["order_key"].copy()
+        for x, y in zip(old, new):
+            a[t["order_key"] == x] = y
+        t["order_key"] = a
+    tc, to, tl = engine.upload("customer", cu), engine.upload("orders", od), engine.upload("lineitem", li)
+    so = to.struct()
+    so.key_max = key_max
+
+    class View:
+        def struct(self):
+            return so
+    try:
+        assert engine.q3(tc, View(), tl.lineitem(80_007 - first, first), k=64) == want
+    finally:
+        for t in (tc, to, tl):
+            engine.free(t)
