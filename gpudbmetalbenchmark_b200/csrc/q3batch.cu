@@ -164,11 +164,12 @@ __global__ void q3m_insert_kernel(Q3Multi m) {
   }
 }
 
+template <int KB>
 __global__ void __launch_bounds__(256) q3m_probe_kernel(const int32_t* __restrict__ lkey, const int32_t* __restrict__ lship,
                                                         const int64_t* __restrict__ lext, const int32_t* __restrict__ ldisc,
                                                         uint64_t n, Q3Multi m) {
-  __shared__ uint32_t scap[kB];
-  __shared__ const uint32_t* sbm[kB];
+  __shared__ uint32_t scap[KB];
+  __shared__ const uint32_t* sbm[KB];
   if (threadIdx.x < (unsigned)m.K) {
     const int r = threadIdx.x;
     scap[r] = m.cnt[4 * r + 1];
@@ -200,30 +201,30 @@ __global__ void __launch_bounds__(256) q3m_probe_kernel(const int32_t* __restric
     // over 6M rows; 165 us so.)
     uint32_t pass = 0, want = 0;   // bit r: request r
 #pragma unroll
-    for (int r = 0; r < kB; r++) {
+    for (int r = 0; r < KB; r++) {
       if (r >= m.K) break;
       const bool p = valid && ship > m.ship_gt[r];
       pass |= (uint32_t)p << r;
       want |= (uint32_t)((__ballot_sync(FULL_MASK, p) & run_mask) != 0u) << r;
     }
     if (!head || key == kEmptyKey) want = 0;
-    uint32_t word[kB];
+    uint32_t word[KB];
 #pragma unroll
-    for (int r = 0; r < kB; r++) {
+    for (int r = 0; r < KB; r++) {
       word[r] = (want >> r) & 1u;
       if (word[r] && sbm[r])
         word[r] = key >= 0 && key <= m.key_max ? __ldg(sbm[r] + ((uint32_t)key >> 5)) >> ((uint32_t)key & 31u) : 0u;
     }
     const uint32_t hash = slot_hash64((uint32_t)key);
-    int32_t slot[kB], home[kB];
+    int32_t slot[KB], home[KB];
 #pragma unroll
-    for (int r = 0; r < kB; r++) {
+    for (int r = 0; r < KB; r++) {
       slot[r] = (word[r] & 1u) ? (int32_t)(hash & (scap[r] - 1)) : -1;
       home[r] = slot[r] >= 0 ? __ldg(&m.ht[(size_t)r * m.max_cap + (uint32_t)slot[r]].key) : 0;
     }
     uint32_t hitbits = 0;   // requests this row joins
 #pragma unroll
-    for (int r = 0; r < kB; r++) {
+    for (int r = 0; r < KB; r++) {
       if (r >= m.K) break;
       if (slot[r] >= 0 && home[r] != key)
         slot[r] = home[r] == kEmptyKey ? -1 : ht_find(m.ht + (size_t)r * m.max_cap, scap[r], key);
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(256) q3m_probe_kernel(const int32_t* __restric
     if (hitbits) {
       const int64_t v = ld_stream(lext + row) * (int64_t)(100 - ld_stream(ldisc + row));
 #pragma unroll
-      for (int r = 0; r < kB; r++) {
+      for (int r = 0; r < KB; r++) {
         if ((hitbits >> r) & 1u) {
           const size_t at = (size_t)r * m.max_cap + (uint32_t)slot[r];
           atomicAdd(&m.ht[at].rev, (unsigned long long)v);
@@ -350,9 +351,10 @@ int q3_batch_run(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32_t
                od.order_date, n_or, cu.key_max, m);
   GPUDB_LAUNCH(call, q3m_clear_kernel, dim3(std::max(1u, grid(max_cap) / 4), K), 256, 0, m);
   GPUDB_LAUNCH(call, q3m_insert_kernel, grid(n_or / 4), 256, 0, m);
+  auto probe = K <= 2 ? q3m_probe_kernel<2> : K <= 4 ? q3m_probe_kernel<4> : q3m_probe_kernel<kB>;
   const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((li.n_rows + 255) / 256, (uint64_t)sms * 8));
   if (li.n_rows)
-    GPUDB_LAUNCH(call, q3m_probe_kernel, g, 256, 0, li.order_key, li.ship_date, li.ext_price, li.discount, li.n_rows, m);
+    GPUDB_LAUNCH(call, probe, g, 256, 0, li.order_key, li.ship_date, li.ext_price, li.discount, li.n_rows, m);
   GPUDB_LAUNCH(call, q3m_hist_kernel, dim3(q3_topk_grid(max_cap, sms, K, 4), K), kTopkThreads, 0, m);
   GPUDB_LAUNCH(call, q3m_select_kernel, dim3(q3_topk_grid(max_cap, sms, K, 2), K), kTopkThreads, 0, m);
   std::vector<uint32_t> idv = ids;

@@ -303,3 +303,28 @@ def test_two_q1_requests_in_one_scan(engine, orc, cuts):
             else:
                 assert r.status == capi.OK and q1_to_dict(o) == orc.q1(li, c), c
         engine.free(t)
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("bounded", [True, False])
+def test_batched_q3_of_every_size(engine, orc, K, bounded):
+    """Groups of Q3 requests of every probe form (up to 2, 4 and 8 requests), with and without a
+    bound on the order keys (no bitmap: every run head walks the tables)."""
+    cu, od, li = orc.q3_tables(3000, 30_000, 120_003, 37)
+    tc, to, tl = engine.upload("customer", cu), engine.upload("orders", od), engine.upload("lineitem", li)
+    so = to.struct()
+    if not bounded:
+        so.key_max = -1
+    tables = capi.Q3Tables(tc.struct(), so, tl.lineitem())
+    cases = [(i % 5, 300 + 250 * i, 2400 - 250 * i, 5 + i) for i in range(K)]
+    reqs, outs = (capi.Request * K)(), [capi.Q3Result() for _ in range(K)]
+    try:
+        for r, o, (seg, d, s, k) in zip(reqs, outs, cases):
+            r.pipeline, r.q3, r.q3_out = capi.PIPE_Q3, C.pointer(tables), C.pointer(o)
+            r.q3p = capi.Q3Params(seg, d, s, k, capi.JOIN_GLOBAL, 0)
+        engine._check(engine.lib.gpudb_batch_run(engine.ctx, reqs, K, None, None))
+        for r, o, c in zip(reqs, outs, cases):
+            assert r.status == capi.OK and q3_to_list(o) == orc.q3(cu, od, li, *c), c
+    finally:
+        for t in (tc, to, tl):
+            engine.free(t)
