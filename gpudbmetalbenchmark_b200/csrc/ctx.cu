@@ -508,6 +508,7 @@ int gpudb_create(int device, gpudb_ctx** out) {
   gpudb_ctx* ctx = new gpudb_ctx();
   ctx->device = device;
   ctx->sm_count = prop.multiProcessorCount;
+  ctx->l2_bytes = (uint64_t)prop.l2CacheSize;
   size_t free_mem = 0;
   cudaError_t e = cudaMemGetInfo(&free_mem, &ctx->total_mem);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);

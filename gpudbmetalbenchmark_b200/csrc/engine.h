@@ -42,6 +42,7 @@ struct gpudb_ctx {
   int device = 0;
   int sm_count = 0;
   size_t total_mem = 0;                // device memory (read once: cudaMemGetInfo takes ~100 us a call)
+  uint64_t l2_bytes = 0;
   cudaStream_t stream = nullptr;       // compute stream
   cudaStream_t copy_stream = nullptr;  // host->device copies of streamed chunks
   cudaStream_t side_stream = nullptr;  // independent stages of one call (Call::side_begin)

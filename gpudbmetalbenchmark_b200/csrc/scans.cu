@@ -77,7 +77,12 @@ __device__ __forceinline__ void block_fold_q6(int64_t rev, uint64_t cnt, int64_t
   }
 }
 
-template <int UNROLL>
+// KEEP: loads that leave the columns in L2 for the next scan of the table (they fit); else loads
+// that do not displace what is there.
+template <bool KEEP, class T>
+__device__ __forceinline__ T q6_load(const T* p) { return KEEP ? __ldg(p) : ld_stream(p); }
+
+template <int UNROLL, bool KEEP>
 __global__ void __launch_bounds__(kThreads) q6_vec_kernel(const int4* __restrict__ ship4, const int4* __restrict__ disc4,
                                                           const int4* __restrict__ qty4, const int64_t* __restrict__ ext,
                                                           uint64_t n, Q6P p, int64_t* part_rev, uint64_t* part_cnt,
@@ -89,16 +94,16 @@ __global__ void __launch_bounds__(kThreads) q6_vec_kernel(const int4* __restrict
   uint32_t cnt = 0;
 #define Q6_ROW(c, j)                                                      \
   if (q6_pass(s.c, d.c, k.c, p)) {                                        \
-    rev += ld_stream(ext + 4 * qq + (j)) * (int64_t)d.c;                  \
+    rev += q6_load<KEEP>(ext + 4 * qq + (j)) * (int64_t)d.c;                  \
     cnt++;                                                                \
   }
   for (; q + (UNROLL - 1) * T < nq; q += UNROLL * T) {
     int4 sv[UNROLL], dv[UNROLL], kv[UNROLL];
 #pragma unroll
     for (int u = 0; u < UNROLL; u++) {
-      sv[u] = ld_stream(ship4 + q + u * T);
-      dv[u] = ld_stream(disc4 + q + u * T);
-      kv[u] = ld_stream(qty4 + q + u * T);
+      sv[u] = q6_load<KEEP>(ship4 + q + u * T);
+      dv[u] = q6_load<KEEP>(disc4 + q + u * T);
+      kv[u] = q6_load<KEEP>(qty4 + q + u * T);
     }
 #pragma unroll
     for (int u = 0; u < UNROLL; u++) {
@@ -109,7 +114,7 @@ __global__ void __launch_bounds__(kThreads) q6_vec_kernel(const int4* __restrict
   }
   for (; q < nq; q += T) {
     const uint64_t qq = q;
-    const int4 s = ld_stream(ship4 + q), d = ld_stream(disc4 + q), k = ld_stream(qty4 + q);
+    const int4 s = q6_load<KEEP>(ship4 + q), d = q6_load<KEEP>(disc4 + q), k = q6_load<KEEP>(qty4 + q);
     Q6_ROW(x, 0) Q6_ROW(y, 1) Q6_ROW(z, 2) Q6_ROW(w, 3)
   }
 #undef Q6_ROW
@@ -838,17 +843,22 @@ int launch_q6(Call& call, const gpudb_lineitem& c, const gpudb_q6_params& p, voi
   const Q6P pp{p.ship_lo, p.ship_hi, p.disc_lo, p.disc_hi, p.qty_lt};
   const bool vec = aligned(c.ship_date, 16) && aligned(c.discount, 16) && aligned(c.quantity, 16) && aligned(c.ext_price, 8);
   // 1 one row per thread; 2/3/4: 128-bit loads, 1/2/4 quads per thread per step. Auto (0): one
-  // quad per step, but one row per thread from 2^21 rows while the columns (20 B a row) fit the
-  // 126 MB L2: over one table that stays there the row form is ahead (6M rows 20.4 us against
-  // 23.2, 3M 22.7 against 23.8 a call), below and above it is not (two tables in turn: 1M rows
-  // 19.0 us against 17.8, 12M 56 against 44)
-  int variant = ctx->q6_variant ? ctx->q6_variant
-                                : (c.n_rows >= (1u << 21) && c.n_rows * 20 <= (126ull << 20) ? 1 : 2);
+  // quad, its loads left in L2 where the columns (20 B a row) would fit; one row while a row a
+  // thread is less than half a wave of blocks. us a call for one row / one
+  // quad / two quads over one table again and again, and over enough tables in turn that none
+  // stays in L2:
+  //   50K rows 15.2 / 15.6 / 16.5; 100K 15.4 / 15.4 / 15.5; 200K 17.1 / 15.8 / 16.5; 1M 17.9 / 17.3 / 16.9 and 20.3 / 19.1 / 19.2
+  //   3M 21.0 / 19.2 / 19.7 and 27.1 / 23.7 / 24.5; 6M 26.5 / 24.4 / 24.5 and 37.2 / 30.9 / 31.9
+  //   8M 41.8 / 35.7 / 36.4; 16M 68 / 53 / 56
+  // (one quad without the loads left in L2: 3M rows 23.6 us over one table, 6M 30.2).
+  const bool keep = c.n_rows * 20 <= ctx->l2_bytes;
+  int variant = ctx->q6_variant ? ctx->q6_variant : c.n_rows < (1u << 17) ? 1 : 2;
   if (!vec) variant = 1;
   const int unroll = variant == 2 ? 1 : variant == 4 ? 4 : 2;
-  const void* kfn = variant == 1 ? (const void*)q6_row_kernel
-                    : unroll == 1 ? (const void*)q6_vec_kernel<1>
-                    : unroll == 4 ? (const void*)q6_vec_kernel<4> : (const void*)q6_vec_kernel<2>;
+  auto kern = unroll == 1 ? (keep ? q6_vec_kernel<1, true> : q6_vec_kernel<1, false>)
+            : unroll == 4 ? (keep ? q6_vec_kernel<4, true> : q6_vec_kernel<4, false>)
+                          : (keep ? q6_vec_kernel<2, true> : q6_vec_kernel<2, false>);
+  const void* kfn = variant == 1 ? (const void*)q6_row_kernel : (const void*)kern;
   const int grid = variant == 1 ? grid_for(ctx, kfn, c.n_rows, 1) : grid_for(ctx, kfn, (c.n_rows / 4 + 1) / unroll, 1);
   void* part = nullptr;
   unsigned* ticket = nullptr;
@@ -857,8 +867,7 @@ int launch_q6(Call& call, const gpudb_lineitem& c, const gpudb_q6_params& p, voi
   int64_t* prev = static_cast<int64_t*>(part);
   uint64_t* pcnt = reinterpret_cast<uint64_t*>(prev + grid);
   if (variant != 1) {
-    auto k = unroll == 1 ? q6_vec_kernel<1> : unroll == 4 ? q6_vec_kernel<4> : q6_vec_kernel<2>;
-    GPUDB_LAUNCH(call, k, grid, kThreads, 0, (const int4*)c.ship_date, (const int4*)c.discount,
+    GPUDB_LAUNCH(call, kern, grid, kThreads, 0, (const int4*)c.ship_date, (const int4*)c.discount,
                  (const int4*)c.quantity, c.ext_price, c.n_rows, pp, prev, pcnt, ticket, (Q6Out*)out, hstatus);
   } else {
     GPUDB_LAUNCH(call, q6_row_kernel, grid, kThreads, 0, c.ship_date, c.discount, c.quantity, c.ext_price, c.n_rows,
@@ -987,7 +996,7 @@ static constexpr Q1SmemKernel<2> kRiding2[kMaxRiders + 1] = {q1_vec_smem_kernel<
 int load_scan_kernels(gpudb_ctx* ctx) {
   for (Q1SmemKernel<1> k : kRiding) GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)k, kQ1AccBytes));
   for (Q1SmemKernel<2> k : kRiding2) GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)k, kQ1AccBytes * 2));
-  for (const void* k : {(const void*)q6_row_kernel, (const void*)q6_vec_kernel<1>}) GPUDB_CUDA(ctx, kernel_smem(ctx, k, 16));
+  for (const void* k : {(const void*)q6_row_kernel, (const void*)q6_vec_kernel<1, false>, (const void*)q6_vec_kernel<1, true>}) GPUDB_CUDA(ctx, kernel_smem(ctx, k, 16));
   return GPUDB_OK;
 }
 

@@ -102,7 +102,7 @@ enum {
                                  8 as 7 with registers for three blocks per SM, 9 as 7 with four
                                  quads per thread per step, 10 as 7 with one quad per step and
                                  four blocks per SM */
-  GPUDB_OPT_Q6_VARIANT = 3,   /* Q6 scan kernel: 0 auto (1 from 2^21 rows while the columns fit L2, else 2), 1 one row per thread,
+  GPUDB_OPT_Q6_VARIANT = 3,   /* Q6 scan kernel: 0 auto (1 below 2^17 rows, else 2), 1 one row per thread,
                                  2/3/4 128-bit loads with 1/2/4 quads (4/8/16 rows) per thread per step */
   GPUDB_OPT_HT_LOAD = 4,      /* largest load of the Q3/Q9 build hash tables, percent: 50 (default) or 25 */
   GPUDB_OPT_RADIX_BITS = 5,   /* Q3 radix mode fan-out (bits) when a call's radix_bits is 0; 0 = from the

@@ -45,6 +45,18 @@ def test_every_q6_variant_matches_oracle(orc, variant):
         assert e.q6(t, 100, 2000, 0, 10, 51) == orc.q6(li, 100, 2000, 0, 10, 51)
 
 
+@pytest.mark.parametrize("n", [(1 << 17) - 1, 1 << 17, (1 << 17) + 3, 6_632_243, 6_632_247])
+def test_q6_at_the_sizes_where_its_form_changes(engine, orc, n):
+    """One row a thread below 2^17 rows, quads from there, loads that keep the columns in L2 up to
+    132,644,864 / 20 rows."""
+    li = orc.lineitem(n, seed=27, cols=("ship_date", "discount", "quantity", "ext_price"))
+    t = engine.upload("lineitem", li)
+    try:
+        assert engine.q6(t, 100, 2000, 0, 10, 51) == orc.q6(li, 100, 2000, 0, 10, 51)
+    finally:
+        engine.free(t)
+
+
 def test_tune_joins_then_results_match_oracle(orc):
     cu, od, l3 = orc.q3_tables(4000, 40_000, 160_000, 12)
     with Engine(0) as e:
