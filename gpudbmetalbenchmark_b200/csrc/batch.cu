@@ -408,12 +408,21 @@ int run_scan_batch(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32
   // Q1 requests on aligned columns go two to a read of the rows (the Q1 kernel with two buckets
   // of sums), up to kRideQ6 Q6 requests riding along on each read: 350 us for two of each over 60M
   // rows, 682 us one by one.
+  // Each such scan is a launch of its own, about 14 us of a small table; the shared passes below take
+  // any number of requests for about 52 us, 68 us when a Q1 request is left over from their pairs.
+  // So below kPairRows rows scans are used while there are at most two (three, for an odd number of
+  // requests), and that many only with few riders: 300K rows, eight Q1 requests 55 us shared
+  // and 84 us in scans, four with four Q6 52 and 63 us, three 69 and 49 us; 2.2M rows, eight 136 and
+  // 108 us, four with four 92 and 76 us.
+  // Q6 requests ride if all do, or all but one, or (large tables) if that saves a Q6 pass: one Q1
+  // with eight Q6 over 3.5M rows takes 95 us with four of them riding, 81 us with none.
   // What is left runs the single-request kernels while it is little (both at the copy peak): up
   // to kSoloQ1 Q1 requests on the same columns, and up to kSoloQ6 Q6 requests of a table
   // without a Q1 pass; more share the passes above, whose per-row work for several requests
   // makes them instruction-bound (over 60M rows a Q1 pass takes about 0.45 ms and a Q6 pass
   // about 0.3 ms, against 0.23 ms for the Q1 kernel and 0.14 ms for the Q6 kernel).
   constexpr size_t kSoloQ1 = 2, kSoloQ6 = 3, kRideQ6 = 4;
+  constexpr uint64_t kPairRows = 1ull << 21;
   struct Riding {
     std::vector<uint32_t> q1, q6;
     gpudb_lineitem view;
@@ -434,14 +443,22 @@ int run_scan_batch(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32
         ++it;
         continue;
       }
+      const size_t scans = (l.size() + 1) / 2, odd = l.size() % 2, n6 = mb.q6.size();
+      const bool small = view.n_rows < kPairRows;
+      if (small && (scans > 2 + odd || (scans == 2 + odd && n6 > 2 + 2 * odd))) {
+        ++it;
+        continue;
+      }
+      size_t ride = std::min(n6, kRideQ6 * scans);
+      if (n6 - ride > 1 && (small || (n6 - ride + kMaxQ6 - 1) / kMaxQ6 == (n6 + kMaxQ6 - 1) / kMaxQ6)) ride = 0;
       std::sort(l.begin(), l.end(),   // neighbours share a pass
                 [&](uint32_t a, uint32_t b) { return reqs[ids[a]].q1.ship_le < reqs[ids[b]].q1.ship_le; });
       for (size_t i = 0; i < l.size(); i += 2) {
         Riding rd;
         rd.view = view;
         rd.q1.assign(l.begin() + i, l.begin() + std::min(l.size(), i + 2));
-        const size_t passes = (l.size() - i + 1) / 2;
-        for (size_t r = std::min(kRideQ6, (mb.q6.size() + passes - 1) / passes); r; r--) {
+        const size_t left = scans - i / 2;
+        for (size_t r = (ride + left - 1) / left; r; r--, ride--) {
           rd.q6.push_back(mb.q6.back());
           mb.q6.pop_back();
         }

@@ -138,8 +138,9 @@ def test_identical_joins_in_one_batch(engine, small):
 
 
 def test_shared_scan_q1_cutoffs_and_q6_mix(engine, orc):
-    """One shared pass: Q1 cutoffs that tie, select nothing and select everything, with
-    more than one pass's worth of Q6 and Q1 requests over the same rows."""
+    """Shared passes (a table too small for scans of two Q1 requests each): Q1 cutoffs that tie,
+    select nothing and select everything, with more than one pass's worth of Q6 and Q1
+    requests over the same rows."""
     li = orc.lineitem(70_001, seed=21)
     s = engine.upload("lineitem", li).lineitem()
     cuts = [-1, 0, 1200, 1200, 2526, 2**31 - 1] + [100 * i for i in range(14)]
@@ -303,6 +304,40 @@ def test_two_q1_requests_in_one_scan(engine, orc, cuts):
             else:
                 assert r.status == capi.OK and q1_to_dict(o) == orc.q1(li, c), c
         engine.free(t)
+
+
+@pytest.mark.parametrize("n,first", [(60_005, 0), (60_005, 1), (60_004, 3), ((1 << 21) - 1, 0), (1 << 21, 0)])
+def test_scan_batches_of_every_route(engine, orc, n, first):
+    """Q1 and Q6 requests on both sides of every line of the batch's routing: scans of two Q1
+    requests with Q6 riding, shared passes, single scans and Q6 passes, on tables below and from
+    2^21 rows and on columns off 16 bytes (which never share a scan)."""
+    li = orc.lineitem(n + first, seed=33)
+    s = engine.upload("lineitem", li)
+    view = s.lineitem(n, first)
+    sub = {k: v[first:] for k, v in li.items()}
+    cuts = [100 + 190 * i for i in range(13)]
+    q6s = [(150 * i, 150 * i + 500, i % 11, min(10, i % 11 + 2), 8 + 2 * i) for i in range(13)]
+    want1 = [orc.q1(sub, c) for c in cuts]
+    want6 = [orc.q6(sub, *p) for p in q6s]
+    mixes = [(1, 0), (1, 4), (1, 5), (1, 6), (1, 12), (2, 0), (2, 4), (2, 5), (2, 9), (3, 0), (3, 8), (3, 12), (4, 0),
+             (4, 2), (4, 3), (4, 4), (5, 0), (5, 4), (5, 5), (5, 12), (6, 0), (7, 7), (8, 8), (13, 13), (0, 1), (0, 3),
+             (0, 4), (0, 8), (0, 13)]
+    try:
+        for n1, n6 in mixes:
+            reqs = (capi.Request * (n1 + n6))()
+            o1, o6 = [capi.Q1Result() for _ in range(n1)], [capi.Q6Result() for _ in range(n6)]
+            for i in range(n1):
+                r = reqs[n1 + n6 - 1 - i]
+                r.pipeline, r.li, r.q1, r.q1_out = capi.PIPE_Q1, C.pointer(view), capi.Q1Params(cuts[i], 0), C.pointer(o1[i])
+            for i in range(n6):
+                r = reqs[i]
+                r.pipeline, r.li, r.q6, r.q6_out = capi.PIPE_Q6, C.pointer(view), capi.Q6Params(*q6s[i]), C.pointer(o6[i])
+            engine._check(engine.lib.gpudb_batch_run(engine.ctx, reqs, n1 + n6, None, None))
+            assert all(r.status == capi.OK for r in reqs), (n1, n6)
+            assert [q1_to_dict(o) for o in o1] == want1[:n1], (n1, n6)
+            assert [(o.revenue, o.rows_matched) for o in o6] == want6[:n6], (n1, n6)
+    finally:
+        engine.free(s)
 
 
 @pytest.mark.parametrize("K", [1, 2, 3, 4, 5, 8, 9])
