@@ -373,14 +373,6 @@ gpudb_lineitem row_view(const gpudb_lineitem& li, uint64_t begin, uint64_t end);
 
 int run_scan_batch(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint32_t>& ids, gpudb_timing* t,
                    const gpudb_exec* ex) {
-  if (!ctx->scan_kernels_loaded) {   // at the context's first scan batch
-    int lrc = load_scan_kernels(ctx);
-    if (lrc) return lrc;
-    GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)scan_pass_kernel<0, kMaxQ6>, pass_smem<0, kMaxQ6>()));
-    GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)scan_pass_kernel<1, kMaxQ6WithQ1>, pass_smem<1, kMaxQ6WithQ1>()));
-    GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)scan_pass_kernel<kMaxQ1, kMaxQ6WithQ1>, pass_smem<kMaxQ1, kMaxQ6WithQ1>()));
-    ctx->scan_kernels_loaded = true;
-  }
   // group by (scan columns, row range); within a group, Q1 requests also share their
   // tax/flag/status columns, so they are sub-grouped by those
   using Key = std::tuple<const void*, const void*, const void*, const void*, uint64_t, uint64_t>;
@@ -735,6 +727,16 @@ void run_host_scans(gpudb_ctx* ctx, gpudb_request* reqs, const std::vector<uint3
 
 
 }  // namespace
+
+int load_batch_kernels(gpudb_ctx* ctx) {
+  const int rc = load_scan_kernels(ctx);
+  if (rc) return rc;
+  GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)scan_pass_kernel<0, kMaxQ6>, pass_smem<0, kMaxQ6>()));
+  GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)scan_pass_kernel<1, kMaxQ6WithQ1>, pass_smem<1, kMaxQ6WithQ1>()));
+  GPUDB_CUDA(ctx, kernel_smem(ctx, (const void*)scan_pass_kernel<kMaxQ1, kMaxQ6WithQ1>, pass_smem<kMaxQ1, kMaxQ6WithQ1>()));
+  return GPUDB_OK;
+}
+
 }  // namespace gpudb
 
 using namespace gpudb;

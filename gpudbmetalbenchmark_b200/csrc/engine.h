@@ -74,7 +74,6 @@ struct gpudb_ctx {
   };
   std::vector<Graph> graphs;
   bool use_graphs = true;              // GPUDB_OPT_GRAPHS
-  bool scan_kernels_loaded = false;    // the kernels of a scan batch (load_scan_kernels)
   uint64_t scratch_gen = 0;            // bumped whenever a scratch buffer is (re)allocated
   uint64_t graph_clock = 0;
   std::unordered_map<std::string, gpudb::Buffer> scratch;

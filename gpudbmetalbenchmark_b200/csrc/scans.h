@@ -24,8 +24,10 @@ int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1
 // Whether launch_q1_riders would share one read of these columns between requests.
 bool q1_shared_ok(const gpudb_ctx* ctx, const gpudb_lineitem& c);
 
-// Loads the scan kernels a batch may use. The runtime loads a kernel at its first use, which would
-// hold up a served stream when a batch first has a new mix of requests.
+// Loads the kernels a scan batch may use. The runtime loads a kernel at its first use (50 to 90 us
+// each), which would hold up a served stream whenever a batch first has a new mix of requests; a
+// server loads them all when it opens (1.3 ms, once per process).
+int load_batch_kernels(gpudb_ctx* ctx);
 int load_scan_kernels(gpudb_ctx* ctx);
 
 // Host result from the kQ1ResultBytes device words of one Q1 scan.

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "scans.h"
 
 namespace {
 
@@ -187,12 +188,15 @@ extern "C" int gpudb_serve_open(const gpudb_serve_config* cfg, gpudb_server** ou
   for (uint32_t i = 0; i < cfg->lanes; i++) {
     gpudb_ctx* c = nullptr;
     int rc = gpudb_create(cfg->device, &c);
+    if (rc == GPUDB_OK) {
+      s->lanes.push_back(c);
+      rc = gpudb::load_batch_kernels(c);
+    }
     if (rc != GPUDB_OK) {
       for (auto* l : s->lanes) gpudb_destroy(l);
       delete s;
       return rc;
     }
-    s->lanes.push_back(c);
   }
   for (size_t i = 0; i < s->lanes.size(); i++) s->workers.emplace_back(&gpudb_server::work, s, i);
   *out = s;
