@@ -207,10 +207,11 @@ int Call::begin(size_t result_bytes, bool defer) {
     direct_ = ctx_->h_slots_dev + (size_t)slot_ * kSlotBytes;
   else if (const int rc = clear(dslot_, 0, kSlotHeader + result_bytes))
     return rc;
-  if (!defer)
+  if (!defer || t_)
     if (const int rc = flush_clears()) return rc;
   if (t_) {
-    // the timed region: the call's fills, kernels and copies
+    // the timed region starts after the result slot is cleared: a pipeline's own fills, its
+    // kernels and copies (a timed call's slot is cleared at once, for the same region in all)
     e0_ = event_get(ctx_);
     e1_ = event_get(ctx_);
     if (!e0_ || !e1_) return fail(ctx_, GPUDB_E_CUDA, "cudaEventCreate failed");

@@ -150,9 +150,9 @@ class Call {
   Call(gpudb_ctx* ctx, const gpudb_exec* ex, gpudb_timing* t);
   ~Call();
   // Acquires a slot; header + payload are zero before the first launch: cleared at once, or
-  // (`defer`) with the fills the pipeline asks for next (clear).
+  // (`defer`, a call without timing) with the fills the pipeline asks for next (clear).
   int begin(size_t result_bytes, bool defer = false);
-  // Fills `bytes` at `p` with the byte `value` before the call's next kernel launch. The fills a
+  // Fills `bytes` at `p` (16-byte aligned: scratch and slots are) with the byte `value` before the call's next kernel launch. The fills a
   // pipeline asks for at its start (its slot's among them) go as one kernel: a memset each took
   // about 1.5 us, five of them in a Q3 call. (A pipeline with no fill of its own clears its slot
   // at once, while the host prepares the launch: deferred, it cost such a call 0.9 us.)

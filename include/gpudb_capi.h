@@ -72,7 +72,8 @@ typedef struct gpudb_exec {
 } gpudb_exec;
 
 /* Timing of one call, filled when the call completes. gpu_ms is measured with CUDA events
- * on the launching stream around all of the call's device work (copies included). */
+ * on the launching stream around all of the call's device work (copies included) but the
+ * clearing of its result slot. */
 typedef struct gpudb_timing {
   double gpu_ms;
   double host_ms;          /* wall time of the call on the host */
