@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(kQ1TmaThreads, 1) q1_tma_kernel(const int32_t*
       q1_row(a, sv.z, kv.z, e23.x, dv.z, tv.z, (f >> 16) & 0xFF, (g >> 16) & 0xFF, ship_le);
       q1_row(a, sv.w, kv.w, e23.y, dv.w, tv.w, f >> 24, g >> 24, ship_le);
     }
+    fence_proxy_async();   // (see the comment at fence_proxy_async)
     __syncthreads();
     if (threadIdx.x == 0 && j + STAGES < mine) issue(j + STAGES);
   }
@@ -588,6 +589,7 @@ __global__ void __launch_bounds__(kQ1TmaThreads, 1) q1_ring_kernel(const int32_t
       q1_row(a, sv.z, kv.z, e23.x, dv.z, tv.z, (f >> 16) & 0xFF, (g >> 16) & 0xFF, ship_le);
       q1_row(a, sv.w, kv.w, e23.y, dv.w, tv.w, f >> 24, g >> 24, ship_le);
     }
+    fence_proxy_async();
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   }
@@ -679,6 +681,7 @@ __global__ void __launch_bounds__(THREADS, 1) q1_ring_smem_kernel(const int32_t*
     const int4 tv = *reinterpret_cast<const int4*>(stg + oTax + 16 * t);
     const uint32_t f = *reinterpret_cast<const uint32_t*>(stg + oFlag + 4 * t);
     const uint32_t g = *reinterpret_cast<const uint32_t*>(stg + oStat + 4 * t);
+    fence_proxy_async();
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);   // the tile is in registers: release the stage
     row(sv.x, kv.x, e01.x, dv.x, tv.x, f & 0xFF, g & 0xFF);

@@ -69,7 +69,9 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
 }
 
 // Orders this thread's earlier shared-memory reads before bulk copies that overwrite the same
-// bytes (issued after a barrier, by any thread).
+// bytes (issued after a barrier, by any thread). Called before that barrier wherever a stage is
+// refilled: a barrier orders the reads with other threads' accesses, not with the copies, and
+// reads whose values are used later may still be outstanding at it (Q13 lost keys so).
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 constexpr uint32_t kMbarPollLimit = 1u << 26;
