@@ -235,14 +235,8 @@ static __global__ void __launch_bounds__(256) clear_ranges_kernel(ClearRanges r)
 
 int Call::clear(void* p, int value, size_t bytes) {
   if (!bytes) return GPUDB_OK;
-  if (clears_.count == ClearRanges::kMax || (reinterpret_cast<uintptr_t>(p) & 15u)) {
-    const int rc = flush_clears();
-    if (rc) return rc;
-  }
-  if (reinterpret_cast<uintptr_t>(p) & 15u) {
-    GPUDB_CUDA(ctx_, cudaMemsetAsync(p, value, bytes, s_));
-    return GPUDB_OK;
-  }
+  if (clears_.count == ClearRanges::kMax)
+    if (const int rc = flush_clears()) return rc;
   const int i = clears_.count++;
   clears_.p[i] = static_cast<unsigned char*>(p);
   clears_.n[i] = bytes;

@@ -1019,12 +1019,8 @@ bool q1_shared_ok(const gpudb_ctx* ctx, const gpudb_lineitem& c) {
 
 int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1_params* q1, void* const* q1out,
                      uint32_t* const* q1status, int n6, const gpudb_q6_params* q6, void* const* q6out) {
-  if (n1 < 1 || n1 > 2 || n6 < 0 || n6 > kMaxRiders || !q1_shared_ok(call.ctx(), c)) {
-    int rc = GPUDB_OK;   // one kernel per request
-    for (int r = 0; !rc && r < n1; r++) rc = launch_q1(call, c, q1[r], q1out[r], q1status[r]);
-    for (int r = 0; !rc && r < n6; r++) rc = launch_q6(call, c, q6[r], q6out[r]);
-    return rc;
-  }
+  if (n1 < 1 || n1 > 2 || n6 < 0 || n6 > kMaxRiders || !q1_shared_ok(call.ctx(), c))
+    return fail(call.ctx(), GPUDB_E_INVALID, "a shared Q1 scan takes 1 or 2 Q1 and up to %d Q6 requests on aligned columns", kMaxRiders);
   Q6Riders rd{};
   for (int r = 0; r < n6; r++) {
     rd.p[r] = Q6P{q6[r].ship_lo, q6[r].ship_hi, q6[r].disc_lo, q6[r].disc_hi, q6[r].qty_lt};

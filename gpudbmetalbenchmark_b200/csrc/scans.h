@@ -15,9 +15,8 @@ constexpr size_t kQ1ResultBytes = 6 * 6 * 16;      // 6 groups x {count, qty, ba
 int launch_q6(Call& call, const gpudb_lineitem& c, const gpudb_q6_params& p, void* out, uint32_t* hstatus = nullptr);
 int launch_q1(Call& call, const gpudb_lineitem& c, const gpudb_q1_params& p, void* out, uint32_t* status = nullptr);
 // One scan for n1 (1 or 2) Q1 requests that also evaluates up to 4 Q6 requests on the rows it reads
-// (one read of the table for all of them); each request adds into its own words and, Q1,
-// reports into its own status word. Falls back to one kernel per request for columns off 16
-// bytes, more requests, or a Q1 kernel variant chosen on the context.
+// (one read of the table for all of them), for columns that q1_shared_ok accepts; each request
+// adds into its own words and, Q1, reports into its own status word.
 int launch_q1_riders(Call& call, const gpudb_lineitem& c, int n1, const gpudb_q1_params* q1, void* const* q1out,
                      uint32_t* const* q1status, int n6, const gpudb_q6_params* q6, void* const* q6out);
 
