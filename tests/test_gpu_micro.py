@@ -124,7 +124,7 @@ def test_radix_partition_large_inputs(engine, orc, bits, n):
 def test_radix_partition_every_block_shape(engine, orc, shape):
     """Every scatter block shape (GPUDB_OPT_RADIX_SHAPE) gives the oracle's stable partition,
     in one pass (10 bits) and in two (13 bits), and the same join count; columns that start
-    off a 16-byte boundary (which the bulk-copy ring cannot stage) give it too."""
+    off a 16-byte boundary (loaded a row at a time) give it too."""
     n = 2_000_003
     keys = orc.gen(8, n, seed=shape, n_orders=n // 3, order_mode=1)
     pay = np.arange(n, dtype=np.int32) * 3
@@ -154,11 +154,10 @@ def test_radix_partition_every_block_shape(engine, orc, shape):
 
 
 @pytest.mark.parametrize("shape", [5, 3])
-def test_radix_join_count_through_the_ring(engine, orc, shape):
-    """Tables large enough that every scatter block walks several sub-tiles through its
-    bulk-copy ring: the join count over 10-bit partitions (unstable, keys only) equals the
-    oracle's, also for a probe side whose length is not a whole number of sub-tiles and
-    starts off a 16-byte boundary (direct loads, no ring)."""
+def test_radix_join_count_many_sub_tiles(engine, orc, shape):
+    """Tables large enough that every scatter block walks several sub-tiles: the join count over
+    10-bit partitions (unstable, keys only) equals the oracle's, also for a probe side whose
+    length is not a whole number of sub-tiles and starts off a 16-byte boundary."""
     nb, npr = 3_000_001, 12_000_017
     b = orc.gen(8, nb, seed=41, n_orders=nb // 2, order_mode=2)
     p = orc.gen(8, npr, seed=42, n_orders=nb // 2, order_mode=1)

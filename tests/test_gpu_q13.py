@@ -201,3 +201,23 @@ def test_q13_first_word_of_one_or_two_letters(engine, orc, w1, w2):
     od = dict(cust_key=rng.integers(-1, 301, n).astype(np.int32), comment=np.array(texts, dtype="S80"))
     cu = dict(cust_key=np.arange(300, dtype=np.int32))
     assert run(engine, cu, od, w1, w2) == orc.q13(cu, od, w1, w2)
+
+
+@pytest.mark.parametrize("w1,w2", [(b"special", b"requests"), (b"pinto", b"beans"), (b"s", b"t")])
+@pytest.mark.parametrize("shift,key_shift", [(0, 1), (1, 0), (4, 0), (8, 3), (2, 2)])
+def test_q13_columns_off_16_bytes(engine, orc, w1, w2, shift, key_shift):
+    """Comments that start `shift` bytes (customer keys: rows) off a 16-byte boundary: no bulk
+    copies, and comments read byte by byte."""
+    cu, od = orc.q13_tables(300, 20_011, 17)
+    tc = engine.upload("customer", cu)
+    text = np.concatenate([np.zeros(shift, np.uint8), np.ascontiguousarray(od["comment"], "S80").view(np.uint8)])
+    keys = np.concatenate([np.full(key_shift, 7, np.int32), od["cust_key"]])
+    dt, dk = engine.to_device(text), engine.to_device(keys)
+    view = _View(capi.Orders(n_rows=len(od["cust_key"]), cust_key=dk + 4 * key_shift, comment=dt + shift, key_max=-1,
+                             cust_key_max=299))
+    try:
+        assert engine.q13(tc, view, w1, w2) == orc.q13(cu, od, w1, w2)
+    finally:
+        engine.free(tc)
+        engine.device_free(dt)
+        engine.device_free(dk)

@@ -105,6 +105,21 @@ def test_q9_streamed_fact_table(engine, orc):
         free_all(engine, ts)
 
 
+@pytest.mark.parametrize("nations", [146, 147, 250])
+def test_q9_more_groups_than_a_block_ranks(engine, orc, nations):
+    """Up to 1024 result groups are ordered by rank, more by a bitonic sort (146 nations and seven years
+    are 1022 groups, 147 are 1029)."""
+    tabs = orc.q9_tables(20_000, 1_000, 100_000, 600_000, 15)
+    tabs[1]["nation"][:] = np.arange(1_000) % nations
+    ts = upload_all(engine, tabs)
+    try:
+        want = orc.q9(*tabs)
+        assert (want[1] > 1024) == (nations > 146)
+        assert engine.q9(*ts) == want
+    finally:
+        free_all(engine, ts)
+
+
 def test_q9_no_flagged_part(engine, orc):
     tabs = orc.q9_tables(2_000, 100, 3_000, 10_000, 5)
     tabs[0]["flag"][:] = 0
