@@ -440,12 +440,15 @@ __global__ void __launch_bounds__(256) q3_quad_kernel(
     }
     uint32_t word[4 * U];
     int32_t slot[4 * U];
-    if (DIRECT) {   // (the words are shifted as they are used: shifted as they load, 30M scattered rows took 71 us, not 60)
+    // The direct form shifts the words as it uses them (a row that does not look up has the word 0).
+    // Whole call, 60M clustered rows half of which pass / 30M scattered rows of which few pass: 362 /
+    // 151 us; 363 / 156 with the words shifted as they load; 389 / 145 with `want` tested again.
+    if (DIRECT) {
 #pragma unroll
       for (int r = 0; r < 4 * U; r++) word[r] = (want >> r & 1u) ? __ldg(okbm + ((uint32_t)key[r] >> 5)) : 0u;
 #pragma unroll
       for (int r = 0; r < 4 * U; r++)
-        slot[r] = ((want >> r & 1u) && (word[r] >> ((uint32_t)key[r] & 31u) & 1u)) ? __ldg(omap + key[r]) : -1;
+        slot[r] = (word[r] >> ((uint32_t)key[r] & 31u) & 1u) ? __ldg(omap + key[r]) : -1;
     } else {
 #pragma unroll
       for (int r = 0; r < 4 * U; r++)
