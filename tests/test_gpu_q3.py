@@ -221,6 +221,26 @@ def test_q3_fact_columns_off_16_bytes(engine, orc, mode, first, n_li):
             engine.free(t)
 
 
+@pytest.mark.parametrize("n_li", [(1 << 20) - 1, 1 << 20, (1 << 20) + 3])
+def test_q3_global_without_an_order_key_bound(engine, orc, n_li):
+    """No bitmap of the order keys: a lane per row below 2^20 fact rows, quads from there."""
+    cu, od, li = orc.q3_tables(5000, 200_000, n_li, 43)
+    tc, to, tl = engine.upload("customer", cu), engine.upload("orders", od), engine.upload("lineitem", li)
+    so = to.struct()
+    so.key_max = -1
+
+    class View:
+        def struct(self):
+            return so
+    try:
+        for d, s in ((1170, 1170), (2400, 100)):
+            got = engine.q3(tc, View(), tl, order_date_lt=d, ship_date_gt=s)
+            assert got == orc.q3(cu, od, li, 1, d, s), (d, s)
+    finally:
+        for t in (tc, to, tl):
+            engine.free(t)
+
+
 @pytest.mark.parametrize("first", [0, 1])
 @pytest.mark.parametrize("key_max", [-1, 0, 12_001])
 def test_q3_global_order_keys_outside_the_bound(engine, orc, first, key_max):
