@@ -741,11 +741,11 @@ __global__ void __launch_bounds__(kQ1SmemThreads, MINB) q1_vec_smem_kernel(const
   for (int i = 0; i < NQ1 * 24; i++) q1_acc[i * T + t] = 0;
   uint32_t bad = 0;
   int64_t rrev[NQ6 > 0 ? NQ6 : 1];
-  // Two Q1 requests: the riders share the row's ext * disc (two riders: 369 us of 60M rows, 389 with a
-  // product each); one Q1 request: a product each is ahead (three riders over 300K rows: 37.9 us
-  // a call, 39.8 shared), and with four riders 64-bit counts are (417 us of 60M rows, 433 with 32
-  // bits, which a thread's rows cannot overflow).
-  constexpr bool kShared = NQ1 > 1;
+  // The riders share the row's ext * disc beside two Q1 requests (two riders: 369 us of 60M rows, 389
+  // with a product each), and a lone rider beside one (6M rows 56 us a call, 58); more beside one
+  // do not (two: 63 us, 64 shared; three over 300K rows: 37.9 us, 39.8), and four count in 64 bits
+  // (417 us of 60M rows, 433 with 32 bits, which a thread's rows cannot overflow).
+  constexpr bool kShared = NQ1 > 1 || NQ6 == 1;
   std::conditional_t<NQ1 == 1 && NQ6 == 4, uint64_t, uint32_t> rcnt[NQ6 > 0 ? NQ6 : 1];
 #pragma unroll
   for (int r = 0; r < NQ6; r++) { rrev[r] = 0; rcnt[r] = 0; }
