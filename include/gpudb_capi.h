@@ -481,10 +481,10 @@ int gpudb_radix_join_pairs(gpudb_ctx* ctx, const int32_t* build_keys, uint64_t n
  * One call runs many requests, each with its own exact result and status:
  *  - Q6/Q1 requests over device-resident tables are grouped by (table, row range): Q1 requests on
  *    aligned columns run two to a scan, with up to 4 Q6 requests evaluated on the rows each scan
- *    reads; up to three Q6 requests left run their own scans, more share passes that read the
- *    rows once for up to 8 of them (Q1 requests on unaligned columns: up to 2 per pass with 4 Q6,
- *    one or two alone their own scans), persistent launches that pull row tiles from a device
- *    queue;
+ *    reads (on tables below 2^21 rows only while that takes few scans); the others share passes
+ *    that read the rows once for up to 2 Q1 with 4 Q6, or for up to 8 Q6, requests, persistent
+ *    launches that pull row tiles from a device queue; one or two Q1 and up to three Q6 requests
+ *    left run their own scans;
  *  - Q6/Q1 requests over the same host-resident table share one chunked copy of it;
  *  - Q3 requests (global mode) over the same tables run in groups of up to 8 that share
  *    every stage's launch and one probe pass over the fact table;
