@@ -616,6 +616,7 @@ typedef struct gpudb_serve_stats {
   uint64_t peak_admitted_bytes;
 } gpudb_serve_stats;
 
+/* Opens the lanes and loads every kernel a scan batch may use (about 1 ms, once per process). */
 int gpudb_serve_open(const gpudb_serve_config* cfg, gpudb_server** out);
 /* Queues a request (caller-owned until it completes). GPUDB_E_BUSY if its predicted
  * footprint alone exceeds the budget, GPUDB_E_CLOSED after close. */
